@@ -117,15 +117,45 @@ struct alignas(16) DevCompactFn
     int    core, asym;
 };
 
-// The groups of a model as a kernel argument (constant bank: warp-uniform
-// loads, no per-thread copy) for the model-specialised symmetry-function
-// kernels; models with more groups run the generic kernels.
-constexpr int kParamGroups = 40;
-struct DevGroupTable
+// One group of the pair kernels (sf_pairs.cuh): the members of a symmetry-
+// function group, or a part of them, as a grid of at most 2 eta x 2 lambda x
+// (integer zeta) values; a group with more etas, lambdas or zetas is cut
+// into several.  Radial groups keep all their members.
+constexpr int kPairLevels = 5;      // zeta slots of the member grid
+struct DevPairGroup
+{
+    int    type;           // 2, 3, 9
+    int    e1, e2;
+    int    cutoffSlot;
+    int    memberBegin, memberCount;
+    int    radialBegin;    // radial groups: their members in DevPairTable::radial
+    int    numEta;
+    int    levels;         // bit k: zeta slot k present
+    int    zeta[kPairLevels];   // zeta of every slot: 1, 2, 4, 8, 16 (power-of-two form) or the group's own
+    float  rc2Test;        // squared cutoff of the FP32 candidate test, rounding error added
+    float  etaScaleF[2], lambdaF[2], eta2F[2];
+    double rc;
+    double etaScale[2];    // -eta 64 / ln 2: argument of the table-driven exponential
+    double eta2[2];        // 2 eta
+    double lambda[2];
+    short  combo[4 * kPairLevels];   // (eta * 2 + lambda) * kPairLevels + slot -> member of the group, -1 if absent
+};
+// A radial member: exp(-eta (r - rs)^2) with scale = -eta 64 / ln 2 (FP32 form -eta / ln 2).
+struct DevRadial
+{
+    double scale, rs, eta2;
+    float  scaleF, rsF, eta2F;
+};
+constexpr int kPairGroups = 48;
+constexpr int kPairRadial = 256;
+struct DevPairTable
 {
     int count;
-    int pad_;
-    DevGroup g[kParamGroups];
+    int maxAngular;        // angular groups of the element that has most
+    int begin[kDevMaxElements + 1];   // groups of every element, radial ones first
+    int memberBegin[kDevMaxElements + 1];
+    DevPairGroup g[kPairGroups];
+    DevRadial radial[kPairRadial];
 };
 
 constexpr int kMaxBases = 4;        // exponential bases per group
@@ -174,9 +204,9 @@ struct DevModel
     int maxRows;
     int normalizeNeurons;
     int sortByDistance;   // an angular group has a cutoff below the largest: stage blocks sorted by r
-    int allFast;          // 0, or the zeta slots (2, 4) when every group is planned (rs = 0 bases) and every
-                          // angular group is on the member grid
-    int powBits;          // binary digits of the largest integer power (eta or zeta) of any member grid
+    int pairForm;         // the pair kernels run the model (DevPairTable): 0 no, 1 every zeta a power of two <= 4,
+                          // 2 <= 16, 3 other integers
+    const double* expTable;   // 2^(j/64), j < 64
     double maxCutoff, maxCutoff2;
     DevElement el[kDevMaxElements];
     DevCutoff cutoff[4];

@@ -227,6 +227,8 @@ void DeviceModel::release()
     cudaFree(compactGroups_);
     cudaFree(compactMembers_);
     cudaFree(compactFns_);
+    cudaFree(expTable_);
+    expTable_ = nullptr;
     compactGroups_ = nullptr;
     compactMembers_ = nullptr;
     compactFns_ = nullptr;
@@ -239,6 +241,138 @@ void DeviceModel::release()
     transIndex_ = nullptr;
 }
 
+namespace {
+
+// Groups of the pair kernels (sf_pairs.cuh) from the symmetry-function
+// groups: the angular ones cut into grids of at most 2 eta x 2 lambda x
+// kPairLevels zeta slots (the pairs are enumerated again for every part).
+// Returns DevModel::pairForm, 0 when the kernels of sf_fast.cuh must run the
+// model: an angular function with a shift or a zeta that is no integer (or
+// beyond powAny's 31), a function listed twice, a Gaussian that leaves the
+// range of the table-driven exponential (2^-1000), or more groups than the
+// kernels' argument holds.
+int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& groups,
+              std::vector<DevMember> const& members, DevPairTable& t)
+{
+    const double log2e = 1.0 / std::log(2.0);
+    bool pow4 = true, pow16 = true;
+    for (DevGroup const& g : groups)
+        for (int q = g.memberBegin; q < g.memberBegin + g.memberCount; ++q)
+        {
+            DevMember const& M = members[q];
+            const double reach = g.rc + std::fabs(M.rs);
+            if (!(M.eta >= 0.0) || M.eta * reach * reach * log2e > 1000.0) return 0;
+            if (g.type == 2) continue;
+            if (M.rs != 0.0 || !M.useIntPow || M.zetaInt < 1 || M.zetaInt > 31) return 0;
+            const int z = M.zetaInt;
+            pow16 = pow16 && (z == 1 || z == 2 || z == 4 || z == 8 || z == 16);
+            // |lambda| > 1: 1 + lambda cos may be negative, and such terms vanish (general form)
+            pow16 = pow16 && std::fabs(M.lambda) <= 1.0;
+            pow4 = pow4 && z <= 4;
+        }
+    const int form = !pow16 ? 3 : pow4 ? 1 : 2;
+    int member = 0, radials = 0;
+    for (int e = 0; e < v.numElements; ++e)
+    {
+        t.begin[e] = t.count;
+        t.memberBegin[e] = member;
+        DevElement const& E = v.el[e];
+        int angular = 0;
+        for (int pass = 0; pass < 2; ++pass)
+            for (int k = E.groupBegin; k < E.groupBegin + E.groupCount; ++k)
+            {
+                DevGroup const& g = groups[k];
+                if ((g.type == 2) != (pass == 0)) continue;
+                member = std::max(member, g.memberBegin + g.memberCount);
+                DevPairGroup p{};
+                p.type = g.type;
+                p.e1 = g.e1;
+                p.e2 = g.e2;
+                p.cutoffSlot = g.cutoffSlot;
+                p.memberBegin = g.memberBegin;
+                p.memberCount = g.memberCount;
+                p.rc = g.rc;
+                // FP32 positions and differences: the squared distance is off by less than
+                // 8 2^-24 of the largest squared distance in the list
+                p.rc2Test = (float)(g.rc * g.rc + 2e-6 * m.maxCutoffRadius * m.maxCutoffRadius);
+                if (g.type == 2)
+                {
+                    if (t.count == kPairGroups || radials + g.memberCount > kPairRadial) return 0;
+                    p.radialBegin = radials;
+                    for (int q = g.memberBegin; q < g.memberBegin + g.memberCount; ++q)
+                    {
+                        DevMember const& M = members[q];
+                        t.radial[radials++] = DevRadial{-64.0 * log2e * M.eta, M.rs, 2.0 * M.eta, (float)(-log2e * M.eta),
+                                                        (float)M.rs, (float)(2.0 * M.eta)};
+                    }
+                    t.g[t.count++] = p;
+                    continue;
+                }
+                std::vector<double> etas, lams;
+                std::vector<int> zetas;
+                auto add = [](auto& list, auto x) {
+                    if (std::find(list.begin(), list.end(), x) == list.end()) list.push_back(x);
+                };
+                for (int q = g.memberBegin; q < g.memberBegin + g.memberCount; ++q)
+                {
+                    add(etas, members[q].eta);
+                    add(lams, members[q].lambda);
+                    add(zetas, members[q].zetaInt);
+                }
+                std::sort(etas.begin(), etas.end());
+                std::sort(zetas.begin(), zetas.end());
+                if (form != 3) zetas = {1, 2, 4, 8, 16};
+                for (size_t a = 0; a < etas.size(); a += 2)
+                    for (size_t l = 0; l < lams.size(); l += 2)
+                        for (size_t z = 0; z < zetas.size(); z += kPairLevels)
+                        {
+                            DevPairGroup c = p;
+                            std::fill(c.combo, c.combo + 4 * kPairLevels, (short)-1);
+                            bool eta[2] = {false, false};
+                            for (int q = 0; q < g.memberCount; ++q)
+                            {
+                                DevMember const& M = members[g.memberBegin + q];
+                                const size_t ia = std::find(etas.begin(), etas.end(), M.eta) - etas.begin();
+                                const size_t il = std::find(lams.begin(), lams.end(), M.lambda) - lams.begin();
+                                const size_t iz = std::find(zetas.begin(), zetas.end(), M.zetaInt) - zetas.begin();
+                                if (ia - a > 1 || il - l > 1 || iz - z >= (size_t)kPairLevels) continue;
+                                short& slot = c.combo[((ia - a) * 2 + (il - l)) * kPairLevels + (iz - z)];
+                                if (slot >= 0) return 0;
+                                slot = (short)q;
+                                eta[ia - a] = true;
+                                c.levels |= 1 << (iz - z);
+                            }
+                            if (!eta[0] && !eta[1]) continue;
+                            for (size_t k2 = 0; k2 < (size_t)kPairLevels; ++k2)
+                                c.zeta[k2] = z + k2 < zetas.size() ? zetas[z + k2] : 1;
+                            c.numEta = a + 1 < etas.size() ? 2 : 1;
+                            for (int k2 = 0; k2 < 2; ++k2)
+                            {
+                                const double x = a + k2 < etas.size() ? etas[a + k2] : 0.0;
+                                c.etaScale[k2] = -64.0 * log2e * x;
+                                c.etaScaleF[k2] = (float)(-log2e * x);
+                                c.eta2[k2] = 2.0 * x;
+                                c.eta2F[k2] = (float)c.eta2[k2];
+                                c.lambda[k2] = l + k2 < lams.size() ? lams[l + k2] : 0.0;
+                                c.lambdaF[k2] = (float)c.lambda[k2];
+                            }
+                            if (t.count == kPairGroups) return 0;
+                            t.g[t.count++] = c;
+                            ++angular;
+                        }
+            }
+        t.maxAngular = std::max(t.maxAngular, angular);
+    }
+    for (int e = v.numElements; e <= kDevMaxElements; ++e)
+    {
+        t.begin[e] = t.count;
+        t.memberBegin[e] = member;
+    }
+    return form;
+}
+
+} // namespace
+
 void DeviceModel::upload(Model const& m)
 {
     if (!m.setupDone) throw std::runtime_error("ERROR: setupGeneric() has not been called.\n");
@@ -249,7 +383,6 @@ void DeviceModel::upload(Model const& m)
     DevModel v{};
     v.numElements = (int)m.elements.size();
     v.normalizeNeurons = m.normalizeNeurons ? 1 : 0;
-    v.allFast = 2;
     v.maxCutoff = m.maxCutoffRadius;
     v.maxCutoff2 = m.maxCutoffRadius * m.maxCutoffRadius;
 
@@ -442,10 +575,7 @@ void DeviceModel::upload(Model const& m)
                 }
                 members.push_back(dm);
             }
-            if (!dg.fast || (dg.type != 2 && (!dg.grid || dg.numBases > 1))) v.allFast = 0;   // one staged base
-            if (dg.grid) v.powBits = std::max(v.powBits, std::max(dg.etaBits, dg.zetaBits));
             if (dg.type != 2 && dg.rc < m.maxCutoffRadius) v.sortByDistance = 1;
-            else if (dg.type != 2 && dg.gridNZ > 2 && v.allFast) v.allFast = 4;
             groups.push_back(dg);
         }
         // compact groups (SymGrpCompRad / SymGrpCompAngw members)
@@ -583,6 +713,8 @@ void DeviceModel::upload(Model const& m)
             else weights.insert(weights.end(), (size_t)t.neurons[l], 0.0);
         }
     }
+    pairTable = DevPairTable{};
+    v.pairForm = planPairs(m, v, groups, members, pairTable);
     v.maxSF = maxSF;
     v.maxRows = maxRows;
     v.numCutoffSlots = (int)slotRc.size();
@@ -640,6 +772,10 @@ void DeviceModel::upload(Model const& m)
     up((void**)&transIndex_, transIndexHost.data(), transIndexHost.size() * sizeof(int));
     up((void**)&compactGroups_, compactGroups.data(), compactGroups.size() * sizeof(DevCompactGroup));
     up((void**)&compactMembers_, compactMembers.data(), compactMembers.size() * sizeof(DevCompactMember));
+    double expTable[64];
+    for (int j = 0; j < 64; ++j) expTable[j] = (double)std::exp2((long double)j / 64);
+    up((void**)&expTable_, expTable, sizeof(expTable));
+    v.expTable = expTable_;
     up((void**)&compactFns_, compactFns.data(), compactFns.size() * sizeof(DevCompactFn));
     v.numCompactGroups = (int)compactGroups.size();
     v.compactTypes = 0;
@@ -654,13 +790,6 @@ void DeviceModel::upload(Model const& m)
     v.compactNarrowStaged = compactNarrowStaged;
     v.compactCols = compactCols;
     v.groups = groups_;
-    groupTable = DevGroupTable{};
-    if (groups.size() <= (size_t)kParamGroups)
-    {
-        groupTable.count = (int)groups.size();
-        std::copy(groups.begin(), groups.end(), groupTable.g);
-    }
-    else v.allFast = 0;   // the specialised kernels read the groups from their argument
     v.members = members_;
     v.scaling = scaling_;
     v.rowTable = rowTable_;
@@ -678,7 +807,8 @@ void DeviceModel::upload(Model const& m)
     mix(compactMembers.data(), compactMembers.size() * sizeof(DevCompactMember));
     mix(compactFns.data(), compactFns.size() * sizeof(DevCompactFn));
     mix(&v.numElements, sizeof(int));
-    mix(&v.allFast, sizeof(int));
+    mix(&pairTable, sizeof(pairTable));
+    mix(&v.pairForm, sizeof(int));
     mix(&v.sortByDistance, sizeof(int));
     mix(v.cutoff, sizeof(v.cutoff));
     fingerprint = h;
@@ -1145,9 +1275,32 @@ void Batch::setPositionsDevice(const double* r)
               "positions D2D");
 }
 
+// Symmetry-function pass (0 values, 1 forces) with first-tier shape `variant`.
+void Batch::symmetryFunctionPass(int pass, int precision, int variant)
+{
+    DevModel const& m = dmodel_.view;
+    DevPairTable const& t = dmodel_.pairTable;
+    if (!m.pairForm)
+    {
+        if (pass == 0) launchSFValues(m, v_, precision, sms_, stream_);
+        else launchSFForces(m, v_, precision, sms_, stream_);
+    }
+    else if (pass == 0)
+    {
+        if (precision == PREC_FP64) launchPairValuesF64(m, t, v_, sms_, stream_, variant);
+        else launchPairValuesF32(m, t, v_, sms_, stream_, variant);
+    }
+    else
+    {
+        if (precision == PREC_FP64) launchPairForcesF64(m, t, v_, sms_, stream_, variant);
+        else launchPairForcesF32(m, t, v_, sms_, stream_, variant);
+    }
+}
+
 // The kernel sequence of one evaluation (Mode::evaluateNNP, Mode.cpp:2029-2077).
 void Batch::record(int flags, int precision, int checkExtrapolation, std::vector<Mark>* marks, int stages)
 {
+    cudaGetLastError();   // an error another library's call left on this thread is not these launches'
     DevModel const& m = dmodel_.view;
     const bool sfOnly = (flags & EVAL_SF_ONLY) != 0;
     const bool forces = (flags & EVAL_FORCES) != 0 && !sfOnly;
@@ -1202,7 +1355,7 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
         // the G pass records its candidate acceptance for the force pass
         v_.candMask = nullptr;
         v_.maskCapacity = 0;
-        if (forces && !stored)
+        if (forces && !stored && !m.pairForm)
         {
             launchMaskOffsets(m, v_, sms_, stream_);
             launches += 4;
@@ -1218,7 +1371,7 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
         }
         else
         {
-            launchSFValues(m, dmodel_.groupTable, v_, precision, sms_, stream_, sfShape_[0][precision]);
+            symmetryFunctionPass(0, precision, sfShape_[0][precision]);
             launches += 2;
             if (m.numCompactGroups > 0) launches += launchCompactValues(m, v_, sms_, stream_);
             mark("sf_values");
@@ -1253,7 +1406,7 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
         }
         else
         {
-            launchSFForces(m, dmodel_.groupTable, v_, precision, sms_, stream_, sfShape_[1][precision]);
+            symmetryFunctionPass(1, precision, sfShape_[1][precision]);
             launches += 2;
             if (m.numCompactGroups > 0) launches += launchCompactForces(m, v_, sms_, stream_);
             mark("sf_forces");
@@ -1408,17 +1561,13 @@ Batch::TuneResult Batch::autotune(int precision, int checkExtrapolation, bool us
         // fill every pass input (neighbour data, dE/dG) once, then time the passes alone
         record(EVAL_FORCES, precision, checkExtrapolation);
         pendingVerify_ = true;
-        DevModel const& m = dmodel_.view;
         cudaEvent_t e0, e1;
         cudaCheck(cudaEventCreate(&e0), "event");
         cudaCheck(cudaEventCreate(&e1), "event");
         for (int pass = 0; pass < 2; ++pass)
             for (int v = 0; v < kSFShapeCount; ++v)
             {
-                auto launch = [&] {
-                    if (pass == 0) launchSFValues(m, dmodel_.groupTable, v_, precision, sms_, stream_, v);
-                    else launchSFForces(m, dmodel_.groupTable, v_, precision, sms_, stream_, v);
-                };
+                auto launch = [&] { symmetryFunctionPass(pass, precision, v); };
                 launch();
                 double best = 1e300;
                 for (int rep = 0; rep < 2; ++rep)

@@ -57,7 +57,7 @@ public:
     ~DeviceModel();
     void upload(Model const& m);
     DevModel view;
-    DevGroupTable groupTable{};          // the groups again, passed by value to the specialised kernels
+    DevPairTable pairTable{};            // the groups of the pair kernels (view.pairForm)
     int maxSF = 0;
     size_t numWeights = 0;               // entries of the flat weight array
     uint64_t fingerprint = 0;            // hash of the evaluation plan (groups, members, cutoffs)
@@ -81,6 +81,7 @@ private:
     DevCompactGroup* compactGroups_ = nullptr;
     DevCompactMember* compactMembers_ = nullptr;
     DevCompactFn* compactFns_ = nullptr;
+    double* expTable_ = nullptr;
 };
 
 struct StructureInput
@@ -270,6 +271,7 @@ private:
     };
     void record(int flags, int precision, int checkExtrapolation, std::vector<Mark>* marks = nullptr,
                 int stages = STAGE_ALL);
+    void symmetryFunctionPass(int pass, int precision, int variant);
     DevStatus readStatus();   // the device status word as it is (synchronises)
     void releaseGraph();
     void releaseAll();

@@ -3,16 +3,14 @@
 
 namespace n2p2b200 {
 
-void launchSFValuesF32(DevModel const& m, DevGroupTable const& gt, BatchView const& b, int sms, cudaStream_t st,
-                       int variant)
+void launchSFValuesF32(DevModel const& m, BatchView const& b, int sms, cudaStream_t st)
 {
-    valuesT<float>(m, gt, b, sms, st, variant);
+    valuesT<float>(m, b, sms, st);
 }
 
-void launchSFForcesF32(DevModel const& m, DevGroupTable const& gt, BatchView const& b, int sms, cudaStream_t st,
-                       int variant)
+void launchSFForcesF32(DevModel const& m, BatchView const& b, int sms, cudaStream_t st)
 {
-    forcesT<float>(m, gt, b, sms, st, variant);
+    forcesT<float>(m, b, sms, st);
 }
 
 } // namespace n2p2b200

@@ -101,22 +101,21 @@ __global__ void kCast64to32(int n, const int64_t* __restrict__ in, int* __restri
 
 // symmetry functions
 void launchCutoffValues(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
-// Symmetry-function passes; `variant` (0 .. kSFShapeCount-1) picks the first
-// tier's (stage capacity, warps per block) in the model-specialised kernels:
-// (128, 4), (160, 4), (192, 2).
+// Symmetry-function passes of the general kernels (sf_fast.cuh).
+void launchSFValues(DevModel const& m, BatchView const& b, int precision, int sms, cudaStream_t st);
+void launchSFForces(DevModel const& m, BatchView const& b, int precision, int sms, cudaStream_t st);
+void launchSFValuesF64(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
+void launchSFForcesF64(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
+void launchSFValuesF32(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
+void launchSFForcesF32(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
+// The same passes for the models of the pair kernels (DevModel::pairForm;
+// sf_pairs.cuh); `variant` (0 .. kSFShapeCount - 1): the first tier's stage
+// capacity, 128, 160 or 192 neighbours.
 constexpr int kSFShapeCount = 3;
-void launchSFValues(DevModel const& m, DevGroupTable const& gt, BatchView const& b, int precision, int sms,
-                    cudaStream_t st, int variant);
-void launchSFForces(DevModel const& m, DevGroupTable const& gt, BatchView const& b, int precision, int sms,
-                    cudaStream_t st, int variant);
-void launchSFValuesF64(DevModel const& m, DevGroupTable const& gt, BatchView const& b, int sms, cudaStream_t st,
-                       int variant);
-void launchSFForcesF64(DevModel const& m, DevGroupTable const& gt, BatchView const& b, int sms, cudaStream_t st,
-                       int variant);
-void launchSFValuesF32(DevModel const& m, DevGroupTable const& gt, BatchView const& b, int sms, cudaStream_t st,
-                       int variant);
-void launchSFForcesF32(DevModel const& m, DevGroupTable const& gt, BatchView const& b, int sms, cudaStream_t st,
-                       int variant);
+void launchPairValuesF64(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
+void launchPairValuesF32(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
+void launchPairForcesF64(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
+void launchPairForcesF32(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
 void launchSFDerivatives(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
 void launchContractStored(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
 

@@ -1,6 +1,7 @@
 // Symmetry-function kernels of the evaluation path (G values and the adjoint
-// force pass), one warp per centre atom; included by one translation unit per
-// precision (k_sf_fast_f64.cu, k_sf_fast_f32.cu).
+// force pass) for the models that the pair kernels (sf_pairs.cuh) do not take,
+// one warp per centre atom; included by one translation unit per precision
+// (k_sf_fast_f64.cu, k_sf_fast_f32.cu).
 //
 // Formulas: SymGrpExpRad::calculate (SymGrpExpRad.cpp:144-239),
 // SymGrpExpAngn::calculate (SymGrpExpAngn.cpp:156-403),
@@ -72,20 +73,6 @@ struct alignas(16) Stage
     int nBelow[4][kDevMaxElements];        // per cutoff slot and element: block entries with r < r_c
 };
 
-// Group gi of the model: the specialised kernels (FAST) read it from the
-// group table argument (warp-uniform constant-bank loads), the generic ones
-// copy it from the model's device array.
-template <int FAST>
-__device__ __forceinline__ DevGroup const& groupOf(DevGroupTable const& gt, DevModel const& model, int gi, DevGroup& scratch)
-{
-    if constexpr (FAST != 0) return gt.g[gi];
-    else
-    {
-        scratch = model.groups[gi];
-        return scratch;
-    }
-}
-
 // A group's base widths and lambda values in the pass's precision (the
 // FP32 copies are the FP64 values rounded once on the host).
 template <typename T>
@@ -113,42 +100,35 @@ struct alignas(16) GridCoef
 };
 
 // Per-group member parameters (shared by all lanes).
-// COMPACT (model-specialised kernels): only what planned radial groups and
-// member grids read.
-// GPASS (model-specialised G pass): only the radial plan (base, pw); the
-// arrays of the force pass and of unplanned members shrink to one entry, so
-// the stage of a warp stays small enough for six blocks of four warps.
-template <typename T, bool COMPACT, bool GPASS = false>
+template <typename T>
 struct Members
 {
-    static constexpr bool kLean = COMPACT && GPASS;
-    static constexpr int kM = kMaxMembers, kC = COMPACT ? 1 : kMaxMembers, kF = kLean ? 1 : kMaxMembers;
-    T cw[kF];                // force pass: dE/dG * factorNorm
-    T eta[kF], rs[kF];
-    int base[kM], pw[kM];
-    T zl[kC], fd[kC], lambda[kC], zeta[kC];
-    int zint[kC], flags[kC];  // flags: 1 intPow, 2 calcExp
-    GridCoef<T> gc[kLean ? 1 : 16];   // member grid: force-pass coefficients per (eta, lambda, zeta) combination
+    T cw[kMaxMembers];       // force pass: dE/dG * factorNorm
+    T eta[kMaxMembers], rs[kMaxMembers];
+    int base[kMaxMembers], pw[kMaxMembers];
+    T zl[kMaxMembers], fd[kMaxMembers], lambda[kMaxMembers], zeta[kMaxMembers];
+    int zint[kMaxMembers], flags[kMaxMembers];  // flags: 1 intPow, 2 calcExp
+    GridCoef<T> gc[16];      // member grid: force-pass coefficients per (eta, lambda, zeta) combination
 };
 
 constexpr int kQueue = 128;  // ring of accepted (owner, partner) pairs waiting for a full warp (< 32 + 64)
 
-template <typename T, int CAP, int FAST>
+template <typename T, int CAP>
 struct ValuesSmem
 {
-    Stage<T, CAP, false, FAST ? 1 : kMaxStagedBases> st;
-    Members<T, FAST != 0, true> mb;
+    Stage<T, CAP, false, kMaxStagedBases> st;
+    Members<T> mb;
     int queue[kQueue];
 };
 
 // h: per staged neighbour, the force the centre's energy puts on it, summed
 // over the atom's triplets in the pass's precision (FP32 in the mixed form,
 // whose final per-atom accumulation, kGatherForces, is FP64).
-template <typename T, int CAP, int FAST>
+template <typename T, int CAP>
 struct ForcesSmem
 {
-    Stage<T, CAP, true, FAST ? 1 : kMaxStagedBases> st;
-    Members<T, FAST != 0> mb;
+    Stage<T, CAP, true, kMaxStagedBases> st;
+    Members<T> mb;
     T h[3][CAP];
     int queue[kQueue];
 };
@@ -349,49 +329,38 @@ __device__ void stageFactors(Stage<T, CAP, DF, NB>& S, DevGroup const& G, int la
     __syncwarp();
 }
 
-template <typename T, bool COMPACT, bool GPASS>
-__device__ void stageMembers(Members<T, COMPACT, GPASS>& mb, DevModel const& model, DevGroup const& G, const double* dEdG,
-                             int lane)
+template <typename T>
+__device__ void stageMembers(Members<T>& mb, DevModel const& model, DevGroup const& G, const double* dEdG, int lane)
 {
-    constexpr bool lean = Members<T, COMPACT, GPASS>::kLean;
     __syncwarp();
     for (int q = lane; q < G.memberCount; q += 32)
     {
         DevMember const& M = model.members[G.memberBegin + q];
-        if constexpr (!lean)
-        {
-            mb.cw[q] = dEdG ? (T)(dEdG[M.sf] * M.factorNorm) : T(0);
-            mb.eta[q] = (T)M.eta;
-            mb.rs[q] = (T)M.rs;
-        }
+        mb.cw[q] = dEdG ? (T)(dEdG[M.sf] * M.factorNorm) : T(0);
+        mb.eta[q] = (T)M.eta;
+        mb.rs[q] = (T)M.rs;
         mb.base[q] = M.expBase;
         mb.pw[q] = M.expPow;
-        if constexpr (!COMPACT)
-        {
-            mb.zl[q] = (T)M.zetaLambda;
-            mb.fd[q] = (T)M.factorDeriv;
-            mb.lambda[q] = (T)M.lambda;
-            mb.zeta[q] = (T)M.zeta;
-            mb.zint[q] = M.zetaInt;
-            mb.flags[q] = (M.useIntPow ? 1 : 0) | (M.calcExp ? 2 : 0);
-        }
+        mb.zl[q] = (T)M.zetaLambda;
+        mb.fd[q] = (T)M.factorDeriv;
+        mb.lambda[q] = (T)M.lambda;
+        mb.zeta[q] = (T)M.zeta;
+        mb.zint[q] = M.zetaInt;
+        mb.flags[q] = (M.useIntPow ? 1 : 0) | (M.calcExp ? 2 : 0);
     }
-    if constexpr (!lean)
+    if (G.grid && dEdG && lane < 16)
     {
-        if (G.grid && dEdG && lane < 16)
+        const int q = G.comboMember[lane];
+        GridCoef<T> cf{};
+        if (q >= 0)
         {
-            const int q = G.comboMember[lane];
-            GridCoef<T> cf{};
-            if (q >= 0)
-            {
-                DevMember const& M = model.members[G.memberBegin + q];
-                const double w = dEdG[M.sf] * M.factorNorm;
-                cf.c[0] = (T)(w * M.zetaLambda);
-                cf.c[1] = (T)(w * M.zetaLambda * M.factorDeriv);
-                cf.c[2] = (T)w;
-            }
-            mb.gc[lane] = cf;
+            DevMember const& M = model.members[G.memberBegin + q];
+            const double w = dEdG[M.sf] * M.factorNorm;
+            cf.c[0] = (T)(w * M.zetaLambda);
+            cf.c[1] = (T)(w * M.zetaLambda * M.factorDeriv);
+            cf.c[2] = (T)w;
         }
+        mb.gc[lane] = cf;
     }
     __syncwarp();
 }
@@ -411,8 +380,8 @@ __device__ __noinline__ T gaussShifted(T eta, T rs, T r1, T r2, T r3, int narrow
     return fexp<T>(-eta * (u * u + v * v + (narrow ? w * w : T(0))));
 }
 
-template <typename T, bool COMPACT, bool GPASS>
-__device__ __forceinline__ T angularPow(T pl, Members<T, COMPACT, GPASS> const& mb, int q)
+template <typename T>
+__device__ __forceinline__ T angularPow(T pl, Members<T> const& mb, int q)
 {
     return (mb.flags[q] & 1) ? powInt<T>(pl, mb.zint[q] - 1) : powReal<T>(pl, mb.zeta[q] - T(1));
 }
@@ -457,30 +426,14 @@ __device__ __forceinline__ void tripletGeometry(Stage<T, CAP, DF, NB> const& S, 
     t.dfcjk = T(0);
 }
 
-// Cutoff types with a kernel instance of their own (CUT template argument);
-// every other type runs the instance with the run-time dispatch.
-constexpr int kCutAny = 0, kCutPoly2 = 6;
-
-// The poly2 instances of the model-specialised kernels also take the integer
-// powers of their member grids as compile-time bounded: at most 2 binary
-// digits with two zeta slots (zeta <= 4, eta multiples <= 3), 4 with four
-// slots (zeta <= 16, multiples <= 15).  Models beyond that run the kCutAny
-// instances (run-time bounds).
-template <int FAST, int CUT>
-__host__ __device__ constexpr int sfPowBits()
-{
-    return CUT == kCutPoly2 ? (FAST == 2 ? 2 : 4) : 0;
-}
-
 // r_jk and its cutoff (narrow groups): FP64 in the FP64 form; in the FP32
 // form the cancellation-free factored polynomials (cutoffFdfF32).
-template <typename T, int CUT = kCutAny>
+template <typename T>
 __device__ __forceinline__ void tripletJK(DevCutoff const& cut, Triplet<T>& t)
 {
     t.rijk = frsqrt<T>(t.rjk2);
     t.rjk = t.rjk2 * t.rijk;
-    if constexpr (CUT == kCutPoly2) cutoffPoly2(cut, t.rjk, t.fcjk, t.dfcjk);
-    else if constexpr (sizeof(T) == 4) cutoffFdfF32(cut, t.rjk, t.fcjk, t.dfcjk);
+    if constexpr (sizeof(T) == 4) cutoffFdfF32(cut, t.rjk, t.fcjk, t.dfcjk);
     else cutoffFdf(cut, t.rjk, t.fcjk, t.dfcjk);
 }
 
@@ -490,35 +443,6 @@ __device__ __forceinline__ void loadTriplet(Stage<T, CAP, DF, NB> const& S, DevC
 {
     tripletGeometry<T, CAP>(S, so, sp, t);
     if (narrow) tripletJK<T>(cut, t);
-}
-
-// ILP triplets per lane at once (model-specialised kernels): entries
-// lane + 32 u, u < ILP, of the queue window [qh, qh + take); a lane past
-// the window repeats the window's first entry (in bounds, finite) and its
-// ok[u] is false.  Each step is written for all u together so independent
-// chains could interleave; the kernels run ILP = 1: two triplets per lane
-// measured 1.5x slower on B200 (the extra live registers cut residency
-// from 16 to 12 warps per SM and spilled in the force pass).
-template <int CUT, typename T, int CAP, bool DF, int NB, int ILP>
-__device__ __forceinline__ void loadTriplets(Stage<T, CAP, DF, NB> const& S, DevCutoff const& cut, bool narrow,
-                                             const int* queue, int qh, int take, int lane, Triplet<T> (&t)[ILP],
-                                             int (&so)[ILP], int (&sp)[ILP], bool (&ok)[ILP])
-{
-#pragma unroll
-    for (int u = 0; u < ILP; ++u)
-    {
-        const int idx = lane + 32 * u;
-        ok[u] = idx < take;
-        const int e = queue[(qh + (ok[u] ? idx : 0)) & (kQueue - 1)];
-        so[u] = entryOwner(e);
-        sp[u] = entryPartner(e);
-        tripletGeometry<T, CAP>(S, so[u], sp[u], t[u]);
-    }
-    if (narrow)
-    {
-#pragma unroll
-        for (int u = 0; u < ILP; ++u) tripletJK<T, CUT>(cut, t[u]);
-    }
 }
 
 // Gaussian bases of a triplet: E_b(rij) E_b(rik) exp(-eta_b rjk^2)
@@ -572,21 +496,16 @@ __device__ __forceinline__ T powUniform(T x, int e)
 
 // The squares x^(2^k), k < bits, that pow_int forms (p[0] = x,
 // p[k] = p[k-1]^2; utility.cpp:292-316), shared by the exponents of one
-// base.  BITS > 0: a compile-time bound on the binary digits of every
-// exponent (exactly BITS - 1 squarings); BITS = 0: the warp-uniform run-time
-// `bits` (<= 5; FP32 then forms every square, FP64 selects).
-template <typename T, int BITS>
+// base, up to the warp-uniform `bits` (<= 5; FP32 forms every square, FP64
+// selects).
+template <typename T>
 __device__ __forceinline__ void powSquares(T x, int bits, T (&p)[5])
 {
     p[0] = x;
 #pragma unroll
     for (int k = 1; k < 5; ++k)
     {
-        if constexpr (BITS > 0)
-        {
-            if (k < BITS) p[k] = p[k - 1] * p[k - 1];
-        }
-        else if constexpr (sizeof(T) == 4) p[k] = p[k - 1] * p[k - 1];
+        if constexpr (sizeof(T) == 4) p[k] = p[k - 1] * p[k - 1];
         else p[k] = (k < bits) ? p[k - 1] * p[k - 1] : T(1);
     }
 }
@@ -594,18 +513,14 @@ __device__ __forceinline__ void powSquares(T x, int bits, T (&p)[5])
 // x^e from its squares in pow_int's multiplication order (1 times the
 // square of each set bit of e, in increasing bit order), e < 2^bits and
 // warp-uniform: the same rounding as powUniform with the squares formed once.
-template <typename T, int BITS>
+template <typename T>
 __device__ __forceinline__ T powFromSquares(T const (&p)[5], int e, int bits)
 {
     T r = (e & 1) ? p[0] : T(1);
 #pragma unroll
     for (int k = 1; k < 5; ++k)
     {
-        if constexpr (BITS > 0)
-        {
-            if (k < BITS && ((e >> k) & 1)) r *= p[k];
-        }
-        else if constexpr (sizeof(T) == 4) r = ((e >> k) & 1) ? r * p[k] : r;
+        if constexpr (sizeof(T) == 4) r = ((e >> k) & 1) ? r * p[k] : r;
         else if (k < bits && ((e >> k) & 1)) r *= p[k];
     }
     return r;
@@ -613,36 +528,36 @@ __device__ __forceinline__ T powFromSquares(T const (&p)[5], int e, int bits)
 
 // The two eta slots' Gaussians of a triplet, E_slot = base^etaPow (one
 // set of squares when both slots use the same staged base).
-template <typename T, int BITS>
+template <typename T>
 __device__ __forceinline__ void gridEtas(T const* bv, DevGroup const& G, T (&vS)[2])
 {
     T p[5];
-    powSquares<T, BITS>(G.etaBase[0] == 0 ? bv[0] : bv[1], G.etaBits, p);
-    vS[0] = powFromSquares<T, BITS>(p, G.etaPow[0], G.etaBits);
-    if (G.etaBase[1] != G.etaBase[0]) powSquares<T, BITS>(G.etaBase[1] == 0 ? bv[0] : bv[1], G.etaBits, p);
-    vS[1] = powFromSquares<T, BITS>(p, G.etaPow[1], G.etaBits);
+    powSquares<T>(G.etaBase[0] == 0 ? bv[0] : bv[1], G.etaBits, p);
+    vS[0] = powFromSquares<T>(p, G.etaPow[0], G.etaBits);
+    if (G.etaBase[1] != G.etaBase[0]) powSquares<T>(G.etaBase[1] == 0 ? bv[0] : bv[1], G.etaBits, p);
+    vS[1] = powFromSquares<T>(p, G.etaPow[1], G.etaBits);
 }
 
 // Member grid, G pass: acc[(eta * 2 + lambda) * STRIDE + zeta] += E_eta * pl^zeta * pfc
 // (pl = 1 + lambda cos; terms with pl <= 0 vanish, SymGrpExpAngn.cpp:295).
-template <typename T, int NZ, int STRIDE, int BITS = 0>
+template <typename T, int NZ, int STRIDE>
 __device__ __forceinline__ void gridValues(T const* bv, DevGroup const& G, T cost, T pfc, T* acc)
 {
     T vS[2];
-    gridEtas<T, BITS>(bv, G, vS);
+    gridEtas<T>(bv, G, vS);
 #pragma unroll
     for (int ls = 0; ls < 2; ++ls)
     {
         const T pl = T(1) + groupLambda<T>(G, ls) * cost;
         const T w = pl > T(0) ? pl * pfc : T(0);
         T q[5];
-        if constexpr (NZ <= 2) powSquares<T, BITS>(pl, G.zetaBits, q);
+        if constexpr (NZ <= 2) powSquares<T>(pl, G.zetaBits, q);
 #pragma unroll
         for (int zs = 0; zs < NZ; ++zs)
         {
             // four zeta slots: the squares per slot (fewer live registers)
             const T pz =
-                (NZ <= 2 ? powFromSquares<T, BITS>(q, G.zetaM1[zs], G.zetaBits) : powUniform<T>(pl, G.zetaM1[zs])) * w;
+                (NZ <= 2 ? powFromSquares<T>(q, G.zetaM1[zs], G.zetaBits) : powUniform<T>(pl, G.zetaM1[zs])) * w;
 #pragma unroll
             for (int es = 0; es < 2; ++es) acc[(es * 2 + ls) * STRIDE + zs] += vS[es] * pz;
         }
@@ -653,25 +568,25 @@ __device__ __forceinline__ void gridValues(T const* bv, DevGroup const& G, T cos
 // accumulated onto T1, T2, T3: with a = E_eta pl^(zeta - 1) per combination,
 // T1 = sum c[0] a, T2 = Uij = Uik = Ujk (rs = 0) = pl sum c[1] a and
 // T3 = pl sum c[2] a (terms with pl <= 0 vanish).
-template <typename T, int NZ, bool COMPACT, int BITS = 0>
-__device__ __forceinline__ void gridForces(T const* bv, DevGroup const& G, Members<T, COMPACT> const& mb, T cost, T& T1, T& T2,
+template <typename T, int NZ>
+__device__ __forceinline__ void gridForces(T const* bv, DevGroup const& G, Members<T> const& mb, T cost, T& T1, T& T2,
                                            T& T3)
 {
     T vS[2];
-    gridEtas<T, BITS>(bv, G, vS);
+    gridEtas<T>(bv, G, vS);
 #pragma unroll
     for (int ls = 0; ls < 2; ++ls)
     {
         const T pl = T(1) + groupLambda<T>(G, ls) * cost;
         const bool valid = pl > T(0);
         T q[5];
-        if constexpr (NZ <= 2) powSquares<T, BITS>(pl, G.zetaBits, q);
+        if constexpr (NZ <= 2) powSquares<T>(pl, G.zetaBits, q);
         T S1 = T(0), S2 = T(0), S3 = T(0);
 #pragma unroll
         for (int zs = 0; zs < NZ; ++zs)
         {
             const T pz1 =
-                valid ? (NZ <= 2 ? powFromSquares<T, BITS>(q, G.zetaM1[zs], G.zetaBits) : powUniform<T>(pl, G.zetaM1[zs]))
+                valid ? (NZ <= 2 ? powFromSquares<T>(q, G.zetaM1[zs], G.zetaBits) : powUniform<T>(pl, G.zetaM1[zs]))
                       : T(0);
 #pragma unroll
             for (int es = 0; es < 2; ++es)
@@ -686,30 +601,6 @@ __device__ __forceinline__ void gridForces(T const* bv, DevGroup const& G, Membe
         T1 += S1;
         T2 += S2 * pl;
         T3 += S3 * pl;
-    }
-}
-
-// gridValues of U triplets (pfc = 0 for a triplet that is not to count:
-// it then adds zeros).
-template <typename T, int NZ, int STRIDE, int U, int BITS>
-__device__ __forceinline__ void gridValuesN(T const (&bv)[U][kMaxStagedBases], DevGroup const& G, T const (&cost)[U],
-                                            T const (&pfc)[U], T* acc)
-{
-#pragma unroll
-    for (int u = 0; u < U; ++u) gridValues<T, NZ, STRIDE, BITS>(bv[u], G, cost[u], pfc[u], acc);
-}
-
-// gridForces of U triplets.
-template <typename T, int NZ, bool COMPACT, int U, int BITS>
-__device__ __forceinline__ void gridForcesN(T const (&bv)[U][kMaxStagedBases], DevGroup const& G,
-                                            Members<T, COMPACT> const& mb, T const (&cost)[U], T (&T1)[U], T (&T2)[U],
-                                            T (&T3)[U])
-{
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-    {
-        T1[u] = T2[u] = T3[u] = T(0);
-        gridForces<T, NZ, COMPACT, BITS>(bv[u], G, mb, cost[u], T1[u], T2[u], T3[u]);
     }
 }
 
@@ -730,33 +621,16 @@ __device__ __forceinline__ bool atomInTier(BatchView const& b, int i, int lower,
 // ---------------------------------------------------------------------------
 // G values
 // ---------------------------------------------------------------------------
-// Blocks per SM the register allocation must allow (measured on the water
-// workloads): the specialised G pass with the poly2 cutoff fits 6 four-warp
-// blocks (<= 80 registers; its lean member stage leaves room in shared
-// memory; FP64 with four zeta slots 5), the FP32 force pass with two zeta
-// slots 5; every other four-warp instance 4, the larger stages 1.
-template <typename T, int WARPS, int FAST, int CUT, bool FORCES>
-constexpr int sfMinBlocks()
+template <typename T, int CAP, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 4 : 1)
+    kSFValuesF(DevModel model, BatchView b, int lower, int flagOverflow)
 {
-    if (WARPS != 4 || FAST == 0 || CUT != 6) return WARPS != 4 ? 1 : 4;
-    if (!FORCES) return (sizeof(T) == 8 && FAST == 4) ? 5 : 6;
-    return (sizeof(T) == 4 && FAST == 2) ? 5 : 4;
-}
-
-template <typename T, int CAP, int WARPS, int FAST, int CUT>
-__global__ void __launch_bounds__(WARPS * 32, (sfMinBlocks<T, WARPS, FAST, CUT, false>()))
-    kSFValuesF(DevModel model, BatchView b, int lower, int flagOverflow, DevGroupTable gt)
-{
-    constexpr int ILP = 1;            // triplets per lane and step (see loadTriplets)
-    constexpr int kStep = 32 * ILP;   // triplets per warp step
     extern __shared__ __align__(16) unsigned char smemRaw[];
-    ValuesSmem<T, CAP, FAST>& SM = reinterpret_cast<ValuesSmem<T, CAP, FAST>*>(smemRaw)[threadIdx.x >> 5];
+    ValuesSmem<T, CAP>& SM = reinterpret_cast<ValuesSmem<T, CAP>*>(smemRaw)[threadIdx.x >> 5];
     auto& S = SM.st;
     auto& mb = SM.mb;
     const int lane = threadIdx.x & 31;
-    // Accumulators per sweep: the member grid of the model (FAST = its zeta
-    // slots) or a chunk of members.
-    constexpr int ACC = FAST ? 4 * FAST : kChunkF;
+    constexpr int ACC = kChunkF;   // accumulators per sweep: the member grid or a chunk of members
     const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
     // the warp's atoms i = warp + k warpsPerGrid, tested 32 at a time (one load per lane instead of a
     // dependent load per atom: the upper tiers take few atoms)
@@ -788,9 +662,8 @@ __global__ void __launch_bounds__(WARPS * 32, (sfMinBlocks<T, WARPS, FAST, CUT, 
             int slot = -1;
             for (int g = 0; g < E.groupCount; ++g)
             {
-                DevGroup scratch;
-                DevGroup const& G = groupOf<FAST>(gt, model, E.groupBegin + g, scratch);
-                const bool fastG = FAST || G.fast;
+                const DevGroup G = model.groups[E.groupBegin + g];
+                const bool fastG = G.fast;
                 if (G.cutoffSlot != slot)
                 {
                     stageCutoff<T, CAP>(S, off, n, G.cutoffSlot, b, lane);
@@ -801,7 +674,7 @@ __global__ void __launch_bounds__(WARPS * 32, (sfMinBlocks<T, WARPS, FAST, CUT, 
                 const T rc = (T)G.rc, rc2 = (T)G.rc2;
                 const DevMember* mem = model.members + G.memberBegin;
                 const bool narrow = (G.type == 3);
-                const bool grid = (G.type != 2) && (FAST || G.grid);
+                const bool grid = (G.type != 2) && G.grid;
                 const int mwiGroup = mwi;
                 for (int m0 = 0; m0 < G.memberCount; m0 += (grid ? G.memberCount : ACC))
                 {
@@ -864,33 +737,16 @@ __global__ void __launch_bounds__(WARPS * 32, (sfMinBlocks<T, WARPS, FAST, CUT, 
                             int p0 = 0;
                             while (true)
                             {
-                                if (qn < kStep && p0 < cnt)   // queue stays below kStep + 64 entries
+                                if (qn < 32 && p0 < cnt)   // queue stays below 32 + 64 entries
                                 {
                                     enqueueCandidates<T, CAP>(S, ph[k], cur, p0, rc, rc2, narrow, SM.queue, qh, qn, lane,
                                                               m0 == 0 ? maskOut : nullptr, nullptr, mwi);
                                     p0 += 64;
                                 }
-                                if (qn >= kStep || (drain && qn > 0))
+                                if (qn >= 32 || (drain && qn > 0))
                                 {
-                                    const int take = min(kStep, qn);
-                                    if constexpr (FAST > 0)
-                                    {
-                                        Triplet<T> t[ILP];
-                                        int so[ILP], sp[ILP];
-                                        bool ok[ILP];
-                                        loadTriplets<CUT, T, CAP>(S, model.cutoff[G.cutoffSlot], narrow, SM.queue, qh, take, lane,
-                                                             t, so, sp, ok);
-                                        T bv[ILP][kMaxStagedBases], cost[ILP], pfc[ILP];
-    #pragma unroll
-                                        for (int u = 0; u < ILP; ++u)
-                                        {
-                                            tripletBases<T, CAP>(S, G, narrow, so[u], sp[u], t[u].rjk2, bv[u]);
-                                            cost[u] = t[u].cost;
-                                            pfc[u] = ok[u] ? t[u].fc1 * t[u].fc2 * t[u].fcjk : T(0);
-                                        }
-                                        gridValuesN<T, FAST, FAST, ILP, sfPowBits<FAST, CUT>()>(bv, G, cost, pfc, acc);
-                                    }
-                                    else if (lane < take)
+                                    const int take = min(32, qn);
+                                    if (lane < take)
                                     {
                                         const int e = SM.queue[(qh + lane) & (kQueue - 1)];
                                         const int so = entryOwner(e), sp = entryPartner(e);
@@ -934,8 +790,7 @@ __global__ void __launch_bounds__(WARPS * 32, (sfMinBlocks<T, WARPS, FAST, CUT, 
     #pragma unroll
                     for (int q = 0; q < ACC; ++q)
                     {
-                        const int c = FAST ? (q / (FAST ? FAST : 1)) * 4 + q % (FAST ? FAST : 1) : q;
-                        const int qq = grid ? (int)G.comboMember[c] : (q < mc ? m0 + q : -1);
+                        const int qq = grid ? (int)G.comboMember[q] : (q < mc ? m0 + q : -1);
                         if (qq >= 0)
                         {
                             double sum = warpSum((double)acc[q]);
@@ -972,90 +827,12 @@ __global__ void __launch_bounds__(WARPS * 32, (sfMinBlocks<T, WARPS, FAST, CUT, 
 // their two contributions to distinct slots; rounds add one after another in
 // a fixed order (deterministic, no atomics).
 
-// One warp step of the force pass over the queue window [qh, qh + take),
-// ILP triplets per lane (model-specialised kernels): lane l evaluates
-// entries l + 32 u.  The self-force sums and the scatter into h keep the
-// one-triplet-per-lane order (entry l before l + 32, and the window's
-// halves scattered one after the other).
-template <typename T, int CAP, int FAST, int CUT, int ILP>
-__device__ __forceinline__ void forcesStepN(Stage<T, CAP, true, 1> const& S, Members<T, true> const& mb, DevGroup const& G,
-                                            DevCutoff const& cut, bool narrow, const int* queue, int qh, int take,
-                                            int lane, T (&h)[3][CAP], T& sfx, T& sfy, T& sfz)
+template <typename T, int CAP, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 4 ? 4 : 1)
+    kSFForcesF(DevModel model, BatchView b, int lower)
 {
-    Triplet<T> t[ILP];
-    int so[ILP], sp[ILP];
-    bool ok[ILP];
-    loadTriplets<CUT, T, CAP>(S, cut, narrow, queue, qh, take, lane, t, so, sp, ok);
-    T bv[ILP][kMaxStagedBases], cost[ILP];
-#pragma unroll
-    for (int u = 0; u < ILP; ++u)
-    {
-        tripletBases<T, CAP>(S, G, narrow, so[u], sp[u], t[u].rjk2, bv[u]);
-        cost[u] = t[u].cost;
-    }
-    T T1[ILP], T2[ILP], T3[ILP];
-    gridForcesN<T, FAST, true, ILP, sfPowBits<FAST, CUT>()>(bv, G, mb, cost, T1, T2, T3);
-    T o[ILP][3], q[ILP][3];
-#pragma unroll
-    for (int u = 0; u < ILP; ++u)
-    {
-        Triplet<T> const& x = t[u];
-        const T dfcr2 = S.dfcr[sp[u]];
-        const T pfc = x.fc1 * x.fc2 * x.fcjk;
-        const T pr1 = x.fc2 * x.fcjk * x.dfcr1;
-        const T pr2 = x.fc1 * x.fcjk * dfcr2;
-        const T pr3 = narrow ? x.fc1 * x.fc2 * x.dfcjk * x.rijk : T(0);
-        const T P1 = pfc * ((x.rinv - x.cost * x.ri1 * x.ri1) * T1[u] - T2[u]) + pr1 * T3[u];
-        const T P2 = pfc * ((x.rinv - x.cost * x.ri2 * x.ri2) * T1[u] - T2[u]) + pr2 * T3[u];
-        const T P3 = narrow ? (pfc * (x.rinv * T1[u] + T2[u]) - pr3 * T3[u]) : (pfc * x.rinv * T1[u]);
-        o[u][0] = P1 * x.x1 + P3 * x.dx3;
-        o[u][1] = P1 * x.y1 + P3 * x.dy3;
-        o[u][2] = P1 * x.z1 + P3 * x.dz3;
-        q[u][0] = P2 * x.x2 - P3 * x.dx3;
-        q[u][1] = P2 * x.y2 - P3 * x.dy3;
-        q[u][2] = P2 * x.z2 - P3 * x.dz3;
-        if (ok[u])
-        {
-            sfx -= P1 * x.x1 + P2 * x.x2;
-            sfy -= P1 * x.y1 + P2 * x.y2;
-            sfz -= P1 * x.z1 + P2 * x.z2;
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < ILP; ++u)
-    {
-        // one conflict-free add per round present in this half of the window
-        const int idx = lane + 32 * u;
-        const bool mine = idx < take;
-        const int rnd = mine ? entryRound(queue[(qh + idx) & (kQueue - 1)]) : -1;
-        const int prevRnd = __shfl_up_sync(kFullMask, rnd, 1);
-        const unsigned heads = __ballot_sync(kFullMask, mine && (lane == 0 || prevRnd != rnd));
-        const int mySub = __popc(heads & ((2u << lane) - 1u)) - 1;
-        const int nSub = __popc(heads);
-        for (int r = 0; r < nSub; ++r)
-        {
-            if (mine && mySub == r)
-            {
-                h[0][so[u]] += o[u][0];
-                h[1][so[u]] += o[u][1];
-                h[2][so[u]] += o[u][2];
-                h[0][sp[u]] += q[u][0];
-                h[1][sp[u]] += q[u][1];
-                h[2][sp[u]] += q[u][2];
-            }
-            __syncwarp();
-        }
-    }
-}
-
-template <typename T, int CAP, int WARPS, int FAST, int CUT>
-__global__ void __launch_bounds__(WARPS * 32, (sfMinBlocks<T, WARPS, FAST, CUT, true>()))
-    kSFForcesF(DevModel model, BatchView b, int lower, DevGroupTable gt)
-{
-    constexpr int ILP = 1;            // triplets per lane and step (see loadTriplets)
-    constexpr int kStep = 32 * ILP;   // triplets per warp step
     extern __shared__ __align__(16) unsigned char smemRaw[];
-    ForcesSmem<T, CAP, FAST>& SM = reinterpret_cast<ForcesSmem<T, CAP, FAST>*>(smemRaw)[threadIdx.x >> 5];
+    ForcesSmem<T, CAP>& SM = reinterpret_cast<ForcesSmem<T, CAP>*>(smemRaw)[threadIdx.x >> 5];
     auto& S = SM.st;
     auto& mb = SM.mb;
     const int lane = threadIdx.x & 31;
@@ -1098,9 +875,8 @@ __global__ void __launch_bounds__(WARPS * 32, (sfMinBlocks<T, WARPS, FAST, CUT, 
                     sfz += (double)gsz;
                     gsx = gsy = gsz = T(0);
                 }
-                DevGroup scratch;
-                DevGroup const& G = groupOf<FAST>(gt, model, E.groupBegin + g, scratch);
-                const bool fastG = FAST || G.fast;
+                const DevGroup G = model.groups[E.groupBegin + g];
+                const bool fastG = G.fast;
                 if (G.cutoffSlot != slot)
                 {
                     stageCutoff<T, CAP>(S, off, n, G.cutoffSlot, b, lane);
@@ -1168,25 +944,11 @@ __global__ void __launch_bounds__(WARPS * 32, (sfMinBlocks<T, WARPS, FAST, CUT, 
                     int p0 = 0;
                     while (true)
                     {
-                        if (qn < kStep && p0 < cnt)   // queue stays below kStep + 64 entries
+                        if (qn < 32 && p0 < cnt)   // queue stays below 32 + 64 entries
                         {
                             enqueueCandidates<T, CAP>(S, ph[k], cur, p0, rc, rc2, narrow, SM.queue, qh, qn, lane,
                                                       nullptr, maskIn, mwi);
                             p0 += 64;
-                        }
-                        if constexpr (FAST > 0)
-                        {
-                            if (qn >= kStep || (drain && qn > 0))
-                            {
-                                const int take = min(kStep, qn);
-                                forcesStepN<T, CAP, FAST, CUT, ILP>(S, mb, G, model.cutoff[G.cutoffSlot], narrow, SM.queue, qh,
-                                                              take, lane, SM.h, gsx, gsy, gsz);
-                                qh = (qh + take) & (kQueue - 1);
-                                qn -= take;
-                                __syncwarp();
-                            }
-                            else if (p0 >= cnt) break;
-                            continue;
                         }
                         if (qn >= 32 || (drain && qn > 0))
                         {

@@ -354,7 +354,7 @@ class Batch:
                                                                    per.ctypes.data_as(_P(ctypes.c_int32))))
         return t.value, per
 
-    SHAPES = ((128, 4), (160, 4), (192, 2))   # (stage capacity, warps per block) per shape index
+    SHAPES = ((128, 4), (160, 4), (192, 4))   # (stage capacity, warps per block) per shape index
 
     def autotune(self, useCache=True):
         """Times the three kernel shapes of both symmetry-function passes (the
