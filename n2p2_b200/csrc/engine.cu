@@ -1365,7 +1365,7 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
         }
         if (stored)
         {
-            launchSFDerivatives(m, v_, sms_, stream_);
+            launchSFDerivatives(m, dmodel_.pairTable, v_, sms_, stream_);
             launches += 2;
             mark("sf_derivatives");
         }

@@ -5,7 +5,8 @@
 //
 //   kSFDerivatives G and dG/dr stored per neighbour row (the Atom::Neighbor::dGdr
 //                  layout of Element::setupSymmetryFunctionMemory,
-//                  Element.cpp:289-311) for callers that read dG/dr.
+//                  Element.cpp:289-311) for callers that read dG/dr: models and
+//                  atoms that k_pair_derivatives.cu does not take.
 //   kContractStored the force contraction of stored dG/dr with dE/dG.
 //   kCutoffValues  f_c and df_c of every neighbour entry.
 //
@@ -421,8 +422,17 @@ void launchCutoffValues(DevModel const& m, BatchView const& b, int sms, cudaStre
     kCutoffValues<<<sms * 16, 256, 0, st>>>(m, b);
 }
 
-void launchSFDerivatives(DevModel const& m, BatchView const& b, int sms, cudaStream_t st)
+void launchSFDerivatives(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st)
 {
+    if (m.pairForm)   // the rest: atoms beyond the pair kernels' stage
+    {
+        launchPairDerivatives(m, gt, b, sms, st);
+        constexpr int kPairCap = 1024;
+        const size_t s = sizeof(NbrStage<double, kBigCap>) * kBigWarps;
+        setSmem(kSFDerivatives<kBigCap, kBigWarps, kPairCap>, s);
+        kSFDerivatives<kBigCap, kBigWarps, kPairCap><<<sms, kBigWarps * 32, s, st>>>(m, b);
+        return;
+    }
     size_t s1 = sizeof(NbrStage<double, kStdCap>) * kStdWarps;
     size_t s2 = sizeof(NbrStage<double, kBigCap>) * kBigWarps;
     setSmem(kSFDerivatives<kStdCap, kStdWarps, -1>, s1);

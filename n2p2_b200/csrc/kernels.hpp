@@ -116,7 +116,9 @@ void launchPairValuesF64(DevModel const& m, DevPairTable const& gt, BatchView co
 void launchPairValuesF32(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
 void launchPairForcesF64(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
 void launchPairForcesF32(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
-void launchSFDerivatives(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
+// G and stored dG/dr (FP64).
+void launchSFDerivatives(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st);
+void launchPairDerivatives(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st);
 void launchContractStored(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
 
 // networks, energies, forces

@@ -4,7 +4,8 @@ there: zeta powers of two up to 4 and 16 and other integers, one to three
 widths, lambda other than +-1 (and beyond 1, where terms vanish), shifted
 radial functions, every kind of cutoff function, angular cutoffs below the
 list's; and for atoms of every tier of the stage (from none to more than 384
-neighbours).
+neighbours); and the stored derivatives
+(k_pair_derivatives.cu) through the forces contracted from them.
 
 Tolerances: those of the other parity tests (energies 1e-10 relative, forces
 1e-10 of the largest component), and for the mixed form its budget of
@@ -101,9 +102,10 @@ def test_forms_and_tiers(form, structures, tmp_path):
         m = H.gpu_mode(d, precision=precision)
         b = m.batch(structures)
         b.setPositions(np.concatenate([s.positions for s in structures]))
-        for shape in range(3):
-            b.setShapes(shape, shape)
-            b.evaluate(forces=True, graph=False)
+        for shape in range(4 if precision == "fp64" else 3):   # 3: with stored dG/dr
+            if shape < 3:
+                b.setShapes(shape, shape)
+            b.evaluate(forces=True, storeDGdr=shape == 3, graph=False)
             E, F = b.energies(), b.forces()
             for k, r in enumerate(ref):
                 f = F[start[k]:start[k + 1]]
