@@ -132,31 +132,47 @@ __global__ void __launch_bounds__(256) kLossSum(const double* __restrict__ lossE
 }
 
 // g_is = -(u_i . dG_is/dr_i + sum_{e = (i -> j)} u_j . dG_is/dr_j): the
-// transpose of the stored-dG/dr force contraction.  Lanes own the rows of an
-// entry (distinct SFs), entries are visited in list order.
-// Atoms [a0, a1) only.  With img, the part of g_imgAtom that comes from the
-// atom's own periodic images (entries with j == i) is also written to
-// img[0..numSF): Mode::calculateForces skips those entries
-// (neighborsUnique.begin() + 1, Mode.cpp:1957) while Training::collectDGdxia
-// (Training.cpp:3604-3615) keeps them.
-// With `list`, atoms list[0..a1) instead of [a0, a1).
+// transpose of the stored-dG/dr force contraction.
+// Atoms [a0, a1) only; with `list`, atoms list[a0..a1).  u is an array [N][3]
+// or, with u null, the unit vector of component unitComp of atom unitAtom.
+// With img, the part of g_imgAtom that comes from the atom's own periodic
+// images (entries with j == i) is also written to img[0..numSF):
+// Mode::calculateForces skips those entries (neighborsUnique.begin() + 1,
+// Mode.cpp:1957) while Training::collectDGdxia (Training.cpp:3604-3615) keeps
+// them.
+// A warp per atom, kAdjointSpan entries at a time with their u_j in shared
+// memory.  Where at most kAdjointFew of 32 entries have u_j != 0 (an
+// observation of one force component: one entry in a hundred) only these are
+// read, lanes over the rows; elsewhere lanes read a row over consecutive
+// entries (coalesced) and the row's sum is one warp reduction per span.
+// Reading every entry with lanes over the rows took 101 us per observation of
+// a 96-384-atom box (100 serial iterations of scattered 24-byte loads) against
+// 5 us, and 275 us for 10 k atoms with dense u against 117 us.
+constexpr int kAdjointSpan = 128, kAdjointFew = 8;
+
 __global__ void __launch_bounds__(kTrainWarps * 32) kSFAdjoint(DevModel model, BatchView b, int a0, int a1,
                                                                const double* __restrict__ u, double* __restrict__ g,
                                                                int imgAtom = -1, double* __restrict__ img = nullptr,
-                                                               const int* __restrict__ list = nullptr)
+                                                               const int* __restrict__ list = nullptr,
+                                                               int unitAtom = -1, int unitComp = 0)
 {
     __shared__ double acc[kTrainWarps][kTrainMaxInput];
     __shared__ double accImg[kTrainWarps][kTrainMaxInput];
-    const int lane = threadIdx.x & 31;
-    double* a = acc[threadIdx.x >> 5];
-    double* ai = accImg[threadIdx.x >> 5];
+    __shared__ double span[kTrainWarps][3][kAdjointSpan];
+    __shared__ signed char spanElem[kTrainWarps][kAdjointSpan];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    double* a = acc[w];
+    double* ai = accImg[w];
     const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
+    auto adjoint = [&](int k, int c) {
+        return u ? u[3 * (size_t)k + c] : (k == unitAtom && c == unitComp ? 1.0 : 0.0);
+    };
     for (int k = a0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); k < a1; k += warpsPerGrid)
     {
         const int i = list ? list[k] : k;
         const int ec = b.elem[i];
         DevElement const& E = model.el[ec];
-        const double ux = u[3 * (size_t)i + 0], uy = u[3 * (size_t)i + 1], uz = u[3 * (size_t)i + 2];
+        const double ux = adjoint(i, 0), uy = adjoint(i, 1), uz = adjoint(i, 2);
         __syncwarp();
         const bool track = img && i == imgAtom;
         for (int s = lane; s < E.numSF; s += 32)
@@ -166,18 +182,80 @@ __global__ void __launch_bounds__(kTrainWarps * 32) kSFAdjoint(DevModel model, B
             ai[s] = 0.0;
         }
         __syncwarp();
-        for (int64_t e = b.nbrOffset[i]; e < b.nbrOffset[i + 1]; ++e)
+        const int64_t end = b.nbrOffset[i + 1];
+        for (int64_t e0 = b.nbrOffset[i]; e0 < end; e0 += kAdjointSpan)
         {
-            const int j = b.nbrJ[e];
-            const int en = b.elem[j];
-            const double vx = u[3 * (size_t)j + 0], vy = u[3 * (size_t)j + 1], vz = u[3 * (size_t)j + 2];
-            const int* table = model.rowTable + E.tableBegin[en];
-            for (int r = lane; r < E.rows[en]; r += 32)
+            bool dense = false;
+            unsigned some[kAdjointSpan / 32];
+#pragma unroll
+            for (int c = 0; c < kAdjointSpan / 32; ++c)
             {
-                const double* p = b.dGdr + ((size_t)r * b.nbrCapacity + e) * 3;
-                const double d = p[0] * vx + p[1] * vy + p[2] * vz;
-                a[table[r]] -= d;
-                if (track && j == i) ai[table[r]] -= d;
+                const int64_t e = e0 + c * 32 + lane;
+                double vx = 0.0, vy = 0.0, vz = 0.0;
+                int en = -1;
+                if (e < end)
+                {
+                    const int j = b.nbrJ[e];
+                    en = b.elem[j];
+                    vx = adjoint(j, 0);
+                    vy = adjoint(j, 1);
+                    vz = adjoint(j, 2);
+                }
+                span[w][0][c * 32 + lane] = vx;
+                span[w][1][c * 32 + lane] = vy;
+                span[w][2][c * 32 + lane] = vz;
+                spanElem[w][c * 32 + lane] = (signed char)en;
+                some[c] = __ballot_sync(kFullMask, vx != 0.0 || vy != 0.0 || vz != 0.0);
+                dense = dense || __popc(some[c]) > kAdjointFew;
+            }
+            __syncwarp();
+            if (dense && !track)
+            {
+                for (int en = 0; en < model.numElements; ++en)
+                {
+                    const int* table = model.rowTable + E.tableBegin[en];
+                    for (int r = 0; r < E.rows[en]; ++r)
+                    {
+                        double d = 0.0;
+#pragma unroll
+                        for (int c = 0; c < kAdjointSpan / 32; ++c)
+                        {
+                            const int q = c * 32 + lane;
+                            if (spanElem[w][q] == en)
+                            {
+                                const double* p = b.dGdr + ((size_t)r * b.nbrCapacity + e0 + q) * 3;
+                                d += p[0] * span[w][0][q] + p[1] * span[w][1][q] + p[2] * span[w][2][q];
+                            }
+                        }
+                        d = warpSum(d);
+                        if (lane == 0) a[table[r]] -= d;
+                    }
+                }
+                __syncwarp();
+                continue;
+            }
+#pragma unroll
+            for (int c = 0; c < kAdjointSpan / 32; ++c)
+            {
+                unsigned todo = some[c];
+                while (todo)
+                {
+                    const int q = c * 32 + __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const int64_t e = e0 + q;
+                    const int en = spanElem[w][q];
+                    const double vx = span[w][0][q], vy = span[w][1][q], vz = span[w][2][q];
+                    const bool image = track && b.nbrJ[e] == i;
+                    const int* table = model.rowTable + E.tableBegin[en];
+                    for (int r = lane; r < E.rows[en]; r += 32)
+                    {
+                        const double* p = b.dGdr + ((size_t)r * b.nbrCapacity + e) * 3;
+                        const double d = p[0] * vx + p[1] * vy + p[2] * vz;
+                        a[table[r]] -= d;
+                        if (image) ai[table[r]] -= d;
+                    }
+                    __syncwarp();
+                }
             }
             __syncwarp();
         }
@@ -209,6 +287,10 @@ struct ParamSmem
 // aStruct; no g means g = 0.  With predPart, the warp's sum of L_i goes to
 // predPart[warp] (the value whose gradient this is).  TANGENT false: g must be
 // null (no tangent is carried; the zero-tangent terms are skipped).
+// Latency-bound (one atom per warp, 200 warps): a warp's first atom stores its
+// slice instead of adding to zeros, along a target's weights, 23.4 -> 17.7 us
+// per energy observation of 96-384 atoms.  (The weights staged in shared memory
+// per block: 21.6 us, not kept.)
 template <bool TANGENT>
 __global__ void __launch_bounds__(kTrainWarps * 32) kParamGrad(DevModel model, BatchView b, int a0, int a1,
                                                                const double* __restrict__ aStruct, double aConst,
@@ -225,15 +307,24 @@ __global__ void __launch_bounds__(kTrainWarps * 32) kParamGrad(DevModel model, B
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
     double* slice = gradPart + (size_t)warp * P;
-    for (int p = lane; p < P; p += 32) slice[p] = 0.0;
     double pred = 0.0;
-    __syncwarp();
+    if (a0 + warp >= a1)
+        for (int p = lane; p < P; p += 32) slice[p] = 0.0;
     for (int k = a0 + warp; k < a1; k += warpsPerGrid)
     {
         const int i = list ? list[k] : k;
         const int ec = b.elem[i];
         DevElement const& E = model.el[ec];
         const int L = E.numLayers;
+        // The warp's first atom stores its gradient (the other elements' parameters are 0), later
+        // ones add to it.
+        const bool first = k == a0 + warp;
+        if (first)
+        {
+            const int p0 = E.wOffset[1], p1 = E.bOffset[L - 1] + E.neurons[L - 1];
+            for (int p = lane; p < P; p += 32)
+                if (p < p0 || p >= p1) slice[p] = 0.0;
+        }
         const double a = aStruct ? aStruct[b.atomStruct[i]] : aConst;
         for (int j = lane; j < E.neurons[0]; j += 32)
         {
@@ -244,16 +335,16 @@ __global__ void __launch_bounds__(kTrainWarps * 32) kParamGrad(DevModel model, B
         for (int l = 1; l < L; ++l)
         {
             const int nin = E.neurons[l - 1], nout = E.neurons[l];
-            const double* W = model.weights + E.wOffset[l];
             const double* bias = model.weights + E.bOffset[l];
             if (lane < nout)
             {
                 double z = bias[lane], zd = 0.0;
-                const double* row = W + (size_t)lane * nin;
+                const double* col = model.weightsT + E.wOffset[l] + lane;   // lanes read consecutive weights
                 for (int j = 0; j < nin; ++j)
                 {
-                    z += row[j] * S.in(l, j);
-                    if (TANGENT) zd += row[j] * S.ind(l, j);
+                    const double wj = col[(size_t)j * nout];
+                    z += wj * S.in(l, j);
+                    if (TANGENT) zd += wj * S.ind(l, j);
                 }
                 double f, f1, f2;
                 activate2(E.activation[l], z, f, f1, f2);
@@ -306,14 +397,22 @@ __global__ void __launch_bounds__(kTrainWarps * 32) kParamGrad(DevModel model, B
                 const double zdb = xdb * S.f1[l][lane];
                 S.zb[lane] = zb;
                 S.zdb[lane] = zdb;
-                double* gw = slice + E.wOffset[l] + (size_t)lane * nin;
-                if (TANGENT)
-                    for (int j = 0; j < nin; ++j) gw[j] += zb * S.in(l, j) + zdb * S.ind(l, j);
-                else
-                    for (int j = 0; j < nin; ++j) gw[j] += zb * S.in(l, j);
-                slice[E.bOffset[l] + lane] += zb;
+                double* gb = slice + E.bOffset[l] + lane;
+                *gb = first ? zb : *gb + zb;
             }
             __syncwarp();
+            // lanes along a target's weights: coalesced
+            for (int k2 = 0; k2 < nout; ++k2)
+            {
+                const double zb = S.zb[k2], zdb = S.zdb[k2];
+                double* gw = slice + E.wOffset[l] + (size_t)k2 * nin;
+                for (int j = lane; j < nin; j += 32)
+                {
+                    const double sum = first ? 0.0 : gw[j];
+                    if (TANGENT) gw[j] = sum + (zb * S.in(l, j) + zdb * S.ind(l, j));
+                    else gw[j] = sum + zb * S.in(l, j);
+                }
+            }
             if (l > 1)
             {
                 if (lane < nin)
@@ -335,16 +434,25 @@ __global__ void __launch_bounds__(kTrainWarps * 32) kParamGrad(DevModel model, B
     if (predPart && lane == 0) predPart[warp] = pred;
 }
 
-// grad[p] = scale * sum over warps w (in order) of gradPart[w][p].
-__global__ void kReduceGrad(const double* __restrict__ gradPart, int warps, int P, double* __restrict__ grad,
-                            double scale = 1.0)
+// grad[p] = sum over warps w of gradPart[w][p] in a fixed order: 8 parameters
+// per block, row r of 128 adds w = r, r + 128, ..., then a tree over the rows.
+// (One thread per parameter over all 4,736 slices took 497 us for 1,058
+// parameters: a thousand threads, each a serial chain of loads; now under 10 us.)
+__global__ void __launch_bounds__(1024) kReduceGrad(const double* __restrict__ gradPart, int warps, int P,
+                                                    double* __restrict__ grad)
 {
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x)
+    __shared__ double part[128][9];
+    const int c = threadIdx.x & 7, r = threadIdx.x >> 3, p = blockIdx.x * 8 + c;
+    double s = 0.0;
+    if (p < P)
+        for (int w = r; w < warps; w += 128) s += gradPart[(size_t)w * P + p];
+    part[r][c] = s;
+    for (int h = 64; h > 0; h >>= 1)
     {
-        double s = 0.0;
-        for (int w = 0; w < warps; ++w) s += gradPart[(size_t)w * P + p];
-        grad[p] = scale == 1.0 ? s : s * scale;
+        __syncthreads();
+        if (r < h) part[r][c] += part[r + h][c];
     }
+    if (r == 0 && p < P) grad[p] = part[0][c];
 }
 
 // Adam (GradientDescent::update, DT_ADAM): m, v moments, step
@@ -490,7 +598,7 @@ void Trainer::step(Batch& batch, const double* energiesPhys, const double* force
     const int blocks = warps_ / kTrainWarps;
     kSFAdjoint<<<blocks, kTrainWarps * 32, 0, st>>>(m, b, 0, N, u_, g_);
     kParamGrad<true><<<blocks, kTrainWarps * 32, 0, st>>>(m, b, 0, N, aStruct_, 0.0, g_, P_, gradPart_, nullptr);
-    kReduceGrad<<<(P_ + tb - 1) / tb, tb, 0, st>>>(gradPart_, warps_, P_, grad_);
+    kReduceGrad<<<(P_ + 7) / 8, 1024, 0, st>>>(gradPart_, warps_, P_, grad_);
     cudaCheck(cudaGetLastError(), "trainer launch");
     if (update)
     {
@@ -553,28 +661,33 @@ void Trainer::syncHostModel(cudaStream_t st)
 
 namespace {
 
-__global__ void kSetEntry(double* p, int64_t k, double v) { p[k] = v; }
-
 // The observation's prediction (sum of the warps' values, fixed order) and
 // error: err = ref - prediction, xi = scale * err (Training.cpp:2879-2898,
 // the force weight at :2910-2923).
 // xi[1] keeps the unscaled sum over a task batch's candidates (accumulate),
 // xi[0] that sum times the scale.
-__global__ void kObsError(const double* __restrict__ predPart, int warps, const double* __restrict__ ref,
-                          int64_t refIndex, double scale, double* __restrict__ xi, double* __restrict__ err,
-                          int accumulate)
+struct ObsError
 {
-    const int lane = threadIdx.x;
+    const double* predPart;
+    const double* ref;
+    int64_t refIndex;
+    double scale;
+    double* xi;
+    double* err;
+};
+
+__device__ __forceinline__ void obsError(ObsError const& o, int warps, int accumulate, int lane)
+{
     double p = 0.0;
-    for (int w = lane; w < warps; w += 32) p += predPart[w];
+    for (int w = lane; w < warps; w += 32) p += o.predPart[w];
     p = warpSum(p);
     if (lane == 0)
     {
-        const double e = ref[refIndex] - p;
-        *err = e;
-        const double sum = accumulate ? xi[1] + e : e;
-        xi[1] = sum;
-        xi[0] = scale == 1.0 ? sum : sum * scale;
+        const double e = o.ref[o.refIndex] - p;
+        *o.err = e;
+        const double sum = accumulate ? o.xi[1] + e : e;
+        o.xi[1] = sum;
+        o.xi[0] = o.scale == 1.0 ? sum : sum * o.scale;
     }
 }
 
@@ -583,11 +696,17 @@ __global__ void kObsError(const double* __restrict__ predPart, int warps, const 
 // row order.  32 parameters x 8 slice rows per block.
 // With `accumulate` the sum is added to out's previous value before scaling
 // (task batches: the candidates' Jacobians are summed, then scaled once).
+// The grid's last block forms the observation's error instead.
 __global__ void __launch_bounds__(256) kReduceSlices(const double* __restrict__ part, int slices, int P,
-                                                     double* __restrict__ out, double scale, int accumulate)
+                                                     double* __restrict__ out, double scale, int accumulate, ObsError o)
 {
     __shared__ double acc[8][32];
     const int lx = threadIdx.x & 31, r = threadIdx.x >> 5;
+    if (blockIdx.x == gridDim.x - 1)
+    {
+        if (r == 0) obsError(o, slices, accumulate, lx);
+        return;
+    }
     const int p = blockIdx.x * 32 + lx;
     double s = 0.0;
     if (p < P)
@@ -1017,7 +1136,6 @@ Training::Training(Model& model, DeviceModel& dmodel, Batch& set, int sms)
     maxWarps_ = (maxWarps_ + kTrainWarps - 1) / kTrainWarps * kTrainWarps;
     eRef_ = tAlloc<double>(S_);
     fRef_ = tAlloc<double>(3 * (size_t)N_);
-    u_ = tAlloc<double>(3 * (size_t)N_);
     g_ = tAlloc<double>((size_t)N_ * b.gStride);
     gradPart_ = tAlloc<double>((size_t)maxWarps_ * P_);
     predPart_ = tAlloc<double>(maxWarps_);
@@ -1037,7 +1155,6 @@ Training::Training(Model& model, DeviceModel& dmodel, Batch& set, int sms)
         colPart_ = tAlloc<double>((size_t)T * (T + 1) / 2 * kTile);
     }
     img_ = tAlloc<double>(b.gStride);
-    cudaCheck(cudaMemsetAsync(u_, 0, sizeof(double) * 3 * (size_t)N_, st), "memset");
     for (int k = 0; k < 2; ++k) cudaCheck(cudaMemsetAsync(Kb_[k], 0, sizeof(double) * P_ * kMaxObs, st), "memset");
     cudaCheck(cudaMemsetAsync(eRef_, 0, sizeof(double) * S_, st), "memset");
     cudaCheck(cudaMemsetAsync(fRef_, 0, sizeof(double) * 3 * (size_t)N_, st), "memset");
@@ -1046,7 +1163,7 @@ Training::Training(Model& model, DeviceModel& dmodel, Batch& set, int sms)
 
 Training::~Training()
 {
-    for (void* p : {(void*)eRef_, (void*)fRef_, (void*)u_, (void*)g_, (void*)gradPart_, (void*)predPart_, (void*)H_,
+    for (void* p : {(void*)eRef_, (void*)fRef_, (void*)g_, (void*)gradPart_, (void*)predPart_, (void*)H_,
                     (void*)xi_, (void*)err_, (void*)Pm_, (void*)Xb_[0], (void*)Xb_[1], (void*)Kb_[0], (void*)Kb_[1], (void*)m_, (void*)v_, (void*)stat_, (void*)singular_, (void*)img_, (void*)rowPart_, (void*)colPart_,
                     (void*)near_})
         cudaFree(p);
@@ -1142,10 +1259,9 @@ void Training::observation(int property, int s, int a, int c, int t, bool accumu
     const int blocks = warps / kTrainWarps;
     if (property == ENERGY)
     {
-        kParamGrad<false><<<blocks, kTrainWarps * 32, 0, st>>>(m, b, a0, a1, nullptr, 1.0, nullptr, P_, gradPart_,
-                                                               predPart_);
-        kReduceSlices<<<(P_ + 31) / 32, 256, 0, st>>>(gradPart_, warps, P_, H, 1.0, acc);
-        kObsError<<<1, 32, 0, st>>>(predPart_, warps, eRef_, s, 1.0, xi, err_ + t, acc);
+        kParamGrad<false><<<blocks, kTrainWarps * 32, 0, st>>>(m, b, a0, a1, nullptr, 1.0, nullptr, P_, gradPart_, predPart_);
+        kReduceSlices<<<(P_ + 31) / 32 + 1, 256, 0, st>>>(gradPart_, warps, P_, H, 1.0, acc,
+                                                          ObsError{predPart_, eRef_, s, 1.0, xi, err_ + t});
     }
     else
     {
@@ -1154,13 +1270,10 @@ void Training::observation(int property, int s, int a, int c, int t, bool accumu
         const int l0 = (int)nearOffset_[a0 + a], l1 = (int)nearOffset_[a0 + a + 1];
         const int fw = std::min(maxWarps_, (l1 - l0 + kTrainWarps - 1) / kTrainWarps * kTrainWarps);
         const int fb = fw / kTrainWarps;
-        kSetEntry<<<1, 1, 0, st>>>(u_, k, 1.0);
-        kSFAdjoint<<<fb, kTrainWarps * 32, 0, st>>>(m, b, l0, l1, u_, g_, a0 + a, img_, near_);
-        kSetEntry<<<1, 1, 0, st>>>(u_, k, 0.0);
-        kParamGrad<true><<<fb, kTrainWarps * 32, 0, st>>>(m, b, l0, l1, nullptr, 0.0, g_, P_, gradPart_, predPart_, a0 + a,
-                                                    img_, near_);
-        kReduceSlices<<<(P_ + 31) / 32, 256, 0, st>>>(gradPart_, fw, P_, H, last ? forceWeight_ : 1.0, acc);
-        kObsError<<<1, 32, 0, st>>>(predPart_, fw, fRef_, k, forceWeight_, xi, err_ + t, acc);
+        kSFAdjoint<<<fb, kTrainWarps * 32, 0, st>>>(m, b, l0, l1, nullptr, g_, a0 + a, img_, near_, a0 + a, c);
+        kParamGrad<true><<<fb, kTrainWarps * 32, 0, st>>>(m, b, l0, l1, nullptr, 0.0, g_, P_, gradPart_, predPart_, a0 + a, img_, near_);
+        kReduceSlices<<<(P_ + 31) / 32 + 1, 256, 0, st>>>(gradPart_, fw, P_, H, last ? forceWeight_ : 1.0, acc,
+                                                          ObsError{predPart_, fRef_, k, forceWeight_, xi, err_ + t});
     }
     cudaCheck(cudaGetLastError(), "observation launch");
 }

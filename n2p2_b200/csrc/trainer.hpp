@@ -185,7 +185,6 @@ private:
     int maxWarps_ = 0;
     double* eRef_ = nullptr;     // [S] internal units
     double* fRef_ = nullptr;     // [3N]
-    double* u_ = nullptr;        // [3N] force adjoint (one unit entry during a force update)
     double* g_ = nullptr;        // [N][gStride]
     double* gradPart_ = nullptr; // [maxWarps][P]
     double* predPart_ = nullptr; // [maxWarps]
