@@ -272,6 +272,8 @@ private:
     void record(int flags, int precision, int checkExtrapolation, std::vector<Mark>* marks = nullptr,
                 int stages = STAGE_ALL);
     void symmetryFunctionPass(int pass, int precision, int variant);
+    void copyPerAtom(const double* dev, double* out);
+    double* packStage_ = nullptr;   // page-locked staging of copyPerAtom, allocated at its first large copy
     DevStatus readStatus();   // the device status word as it is (synchronises)
     void releaseGraph();
     void releaseAll();
