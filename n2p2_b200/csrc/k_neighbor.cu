@@ -59,8 +59,13 @@ __device__ __forceinline__ double norm2Exact(double x, double y, double z)
 // Atom::toNormalizedUnits' r *= convLength (Atom.cpp:78-85).
 __global__ void kPreparePositions(int N, const int* __restrict__ atomStruct, const DevStructInfo* __restrict__ info,
                                   const double* __restrict__ rin, double* __restrict__ px, double* __restrict__ py,
-                                  double* __restrict__ pz, int doRemap, int doNormalize, double convLength)
+                                  double* __restrict__ pz, int doRemap, int doNormalize, double convLength,
+                                  int numCells, int* __restrict__ cellCount, DevStatus* __restrict__ status)
 {
+    // the evaluation's status word and the cells' counts start at 0 (memset nodes between a graph's
+    // kernels would cost a node each)
+    if (blockIdx.x == 0 && threadIdx.x == 0) *status = DevStatus{};
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < numCells; c += gridDim.x * blockDim.x) cellCount[c] = 0;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x)
     {
         DevStructInfo const& s = info[atomStruct[i]];
@@ -599,14 +604,14 @@ void launchPreparePositions(BatchView const& b, const double* rin, int doRemap, 
 {
     int blocks = (b.N + 255) / 256;
     kPreparePositions<<<blocks > 0 ? blocks : 1, 256, 0, st>>>(b.N, b.atomStruct, b.info, rin, b.px, b.py, b.pz,
-                                                               doRemap, doNormalize, convLength);
+                                                               doRemap, doNormalize, convLength, b.numCells, b.cellCount,
+                                                               b.status);
 }
 
 void launchNeighborBuild(BatchView const& b, double rc2, cudaStream_t st)
 {
     const int N = b.N;
     const int blocks = (N + 255) / 256 > 0 ? (N + 255) / 256 : 1;
-    cudaMemsetAsync(b.cellCount, 0, sizeof(int) * (size_t)b.numCells, st);
     kAssignCells<<<blocks, 256, 0, st>>>(N, b.atomStruct, b.info, b.px, b.py, b.pz, b.atomCell, b.atomSlot,
                                          b.cellCount);
     launchExclusiveScan(b.numCells, b.cellCount, b.cellStart64, b.scanTmp, nullptr, st);

@@ -183,12 +183,11 @@ namespace {
 // Tiled FP64 networks: one block per tile of TILE (32, or 16 for wide networks) atoms of one element
 // (element-grouped atom list).  Activations, derivatives and the reverse
 // pass's vectors live in shared memory neuron-major ([neuron][atom], rows of
-// netRow doubles); each thread computes a unit of kNetUnit atoms x one
+// netRow doubles); each thread computes a unit of UNIT atoms x one
 // neuron, reading a weight once (through the read-only cache: every block of
-// an element reads the same matrices) for kNetUnit fused multiply-adds.  Every sum
+// an element reads the same matrices) for UNIT fused multiply-adds.  Every sum
 // runs over the reduction index in ascending order, as in propagateLayer.
 constexpr int kNetThreads = 128;
-constexpr int kNetUnit = 8;        // atoms per thread unit (independent sums)
 
 // Row of a tile of TILE atoms: padded by four against bank conflicts (rows stay 32-byte aligned).
 template <int TILE>
@@ -202,19 +201,19 @@ __host__ __device__ inline int netSmemDoubles(DevElement const& E, int row)
     return (2 * maxW + sumD + 2 * maxW) * row;   // activations, derivatives per layer, reverse vectors
 }
 
-// Sum over the reduction index r < n of w(r) x[r][a] for the unit's kNetUnit
+// Sum over the reduction index r < n of w(r) x[r][a] for the unit's UNIT
 // atoms (x rows ROW apart), in ascending r.
-template <int ROW, typename WF>
-__device__ __forceinline__ void netUnitSums(int n, WF w, const double* x, double (&v)[kNetUnit])
+template <int ROW, int UNIT, typename WF>
+__device__ __forceinline__ void netUnitSums(int n, WF w, const double* x, double (&v)[UNIT])
 {
 #pragma unroll
-    for (int c = 0; c < kNetUnit; ++c) v[c] = 0.0;
+    for (int c = 0; c < UNIT; ++c) v[c] = 0.0;
 #pragma unroll 4
     for (int r = 0; r < n; ++r)
     {
         const double wr = w(r);
 #pragma unroll
-        for (int c = 0; c < kNetUnit; c += 2)
+        for (int c = 0; c < UNIT; c += 2)
         {
             const double2 p = *reinterpret_cast<const double2*>(x + r * ROW + c);
             v[c] += wr * p.x;
@@ -224,51 +223,51 @@ __device__ __forceinline__ void netUnitSums(int n, WF w, const double* x, double
 }
 
 // out[k][a] = act(sum_j W[k][j] in[j][a] + b[k]) (normalize: x / nin), with f' kept.
-template <int TILE>
+template <int TILE, int UNIT>
 __device__ __forceinline__ void netForwardLayer(int af, int nin, int nout, const double* __restrict__ WT,
                                                 const double* __restrict__ bias, int normalize, const double* in,
                                                 double* out, double* df, int tid)
 {
-    for (int u = tid; u < (TILE / kNetUnit) * nout; u += kNetThreads)
+    for (int u = tid; u < (TILE / UNIT) * nout; u += kNetThreads)
     {
         const int k = u % nout, q = u / nout;
-        double v[kNetUnit];
-        netUnitSums<netRow<TILE>()>(nin, [&](int j) { return __ldg(&WT[(size_t)j * nout + k]); }, in + kNetUnit * q, v);
+        double v[UNIT];
+        netUnitSums<netRow<TILE>(), UNIT>(nin, [&](int j) { return __ldg(&WT[(size_t)j * nout + k]); }, in + UNIT * q, v);
         const double bk = __ldg(&bias[k]);
 #pragma unroll
-        for (int c = 0; c < kNetUnit; ++c)
+        for (int c = 0; c < UNIT; ++c)
         {
             double x = v[c] + bk;
             if (normalize) x /= nin;
             double y, dy;
             activate(af, x, y, dy);
-            out[k * netRow<TILE>() + kNetUnit * q + c] = y;
-            df[k * netRow<TILE>() + kNetUnit * q + c] = dy;
+            out[k * netRow<TILE>() + UNIT * q + c] = y;
+            df[k * netRow<TILE>() + UNIT * q + c] = dy;
         }
     }
 }
 
 // out[j][a] = scale[j][a] * sum_k W[k][j] g[k][a] (divided by div when > 0).
-template <int TILE>
+template <int TILE, int UNIT>
 __device__ __forceinline__ void netBackwardLayer(int nin, int nout, const double* __restrict__ W, const double* g,
                                                  const double* scale, int div, double* out, int tid)
 {
-    for (int u = tid; u < (TILE / kNetUnit) * nin; u += kNetThreads)
+    for (int u = tid; u < (TILE / UNIT) * nin; u += kNetThreads)
     {
         const int j = u % nin, q = u / nin;
-        double v[kNetUnit];
-        netUnitSums<netRow<TILE>()>(nout, [&](int k) { return __ldg(&W[(size_t)k * nin + j]); }, g + kNetUnit * q, v);
+        double v[UNIT];
+        netUnitSums<netRow<TILE>(), UNIT>(nout, [&](int k) { return __ldg(&W[(size_t)k * nin + j]); }, g + UNIT * q, v);
 #pragma unroll
-        for (int c = 0; c < kNetUnit; ++c)
+        for (int c = 0; c < UNIT; ++c)
         {
-            double x = v[c] * scale[j * netRow<TILE>() + kNetUnit * q + c];
+            double x = v[c] * scale[j * netRow<TILE>() + UNIT * q + c];
             if (div > 0) x /= div;
-            out[j * netRow<TILE>() + kNetUnit * q + c] = x;
+            out[j * netRow<TILE>() + UNIT * q + c] = x;
         }
     }
 }
 
-template <int TILE>
+template <int TILE, int UNIT>
 __global__ void __launch_bounds__(kNetThreads, 3) kNetworkTiled(DevModel model, BatchView b, int derivatives)
 {
     extern __shared__ __align__(16) unsigned char smemRaw[];
@@ -313,7 +312,7 @@ __global__ void __launch_bounds__(kNetThreads, 3) kNetworkTiled(DevModel model, 
         for (int l = 1; l < L; ++l)
         {
             dfOf[l] = df;
-            netForwardLayer<TILE>(E.activation[l], E.neurons[l - 1], E.neurons[l], model.weightsT + E.wOffset[l],
+            netForwardLayer<TILE, UNIT>(E.activation[l], E.neurons[l - 1], E.neurons[l], model.weightsT + E.wOffset[l],
                             model.weights + E.bOffset[l], model.normalizeNeurons, act[cur], act[cur ^ 1], df, tid);
             df += E.neurons[l] * netRow<TILE>();
             __syncthreads();
@@ -332,7 +331,7 @@ __global__ void __launch_bounds__(kNetThreads, 3) kNetworkTiled(DevModel model, 
         int gc = 0;
         for (int l = L - 1; l >= 2; --l)
         {
-            netBackwardLayer<TILE>(E.neurons[l - 1], E.neurons[l], model.weights + E.wOffset[l], gv[gc], dfOf[l - 1],
+            netBackwardLayer<TILE, UNIT>(E.neurons[l - 1], E.neurons[l], model.weights + E.wOffset[l], gv[gc], dfOf[l - 1],
                              model.normalizeNeurons ? E.neurons[l - 2] : 0, gv[gc ^ 1], tid);
             __syncthreads();
             gc ^= 1;
@@ -340,15 +339,15 @@ __global__ void __launch_bounds__(kNetThreads, 3) kNetworkTiled(DevModel model, 
         // dE/dG into the atoms' rows (rows of atoms beyond the element are not written)
         const int nout1 = E.neurons[1];
         const double* W1 = model.weights + E.wOffset[1];
-        for (int u = tid; u < (TILE / kNetUnit) * nin0; u += kNetThreads)
+        for (int u = tid; u < (TILE / UNIT) * nin0; u += kNetThreads)
         {
             const int j = u % nin0, q = u / nin0;
-            double v[kNetUnit];
-            netUnitSums<netRow<TILE>()>(nout1, [&](int k) { return __ldg(&W1[(size_t)k * nin0 + j]); }, gv[gc] + kNetUnit * q, v);
+            double v[UNIT];
+            netUnitSums<netRow<TILE>(), UNIT>(nout1, [&](int k) { return __ldg(&W1[(size_t)k * nin0 + j]); }, gv[gc] + UNIT * q, v);
 #pragma unroll
-            for (int c = 0; c < kNetUnit; ++c)
-                if (kNetUnit * q + c < count)
-                    b.dEdG[(size_t)b.elemAtoms[first + kNetUnit * q + c] * b.gStride + j] = v[c];
+            for (int c = 0; c < UNIT; ++c)
+                if (UNIT * q + c < count)
+                    b.dEdG[(size_t)b.elemAtoms[first + UNIT * q + c] * b.gStride + j] = v[c];
         }
         __syncthreads();
     }
@@ -357,18 +356,45 @@ __global__ void __launch_bounds__(kNetThreads, 3) kNetworkTiled(DevModel model, 
 } // namespace
 
 // E_s = sum of atomic energies of structure s (Mode::calculateEnergy,
-// Mode.cpp:1876-1901), one warp per structure, fixed summation order.
-__global__ void kEnergySum(BatchView b)
+// Mode.cpp:1876-1901), one warp per structure, fixed summation order; a
+// structure of more than kEnergyWarpAtoms atoms by its whole block (110,592
+// atoms: 126 us by one warp, 14 by the block).  The order depends on the
+// structure alone, not on the batch.
+constexpr int kEnergyWarpAtoms = 4096;
+
+__global__ void __launch_bounds__(256) kEnergySum(BatchView b)
 {
-    const int lane = threadIdx.x & 31;
-    const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
-    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < b.S; s += warpsPerGrid)
+    __shared__ double part[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int s0 = blockIdx.x * 8, s1 = min(s0 + 8, b.S);
+    if (s0 + warp < s1)
+    {
+        const int s = s0 + warp;
+        const int a0 = b.structAtomBegin[s], a1 = b.structAtomBegin[s + 1];
+        if (a1 - a0 <= kEnergyWarpAtoms)
+        {
+            double e = 0.0;
+            for (int a = a0 + lane; a < a1; a += 32) e += b.Eatom[a];
+            e = warpSum(e);
+            if (lane == 0) b.Estruct[s] = e;
+        }
+    }
+    for (int s = s0; s < s1; ++s)
     {
         const int a0 = b.structAtomBegin[s], a1 = b.structAtomBegin[s + 1];
+        if (a1 - a0 <= kEnergyWarpAtoms) continue;
         double e = 0.0;
-        for (int a = a0 + lane; a < a1; a += 32) e += b.Eatom[a];
+#pragma unroll 8
+        for (int a = a0 + (int)threadIdx.x; a < a1; a += 256) e += b.Eatom[a];
         e = warpSum(e);
-        if (lane == 0) b.Estruct[s] = e;
+        __syncthreads();
+        if (lane == 0) part[warp] = e;
+        __syncthreads();
+        if (threadIdx.x == 0)
+        {
+            for (int w = 1; w < 8; ++w) e += part[w];
+            b.Estruct[s] = e;
+        }
     }
 }
 
@@ -559,13 +585,15 @@ void launchExtrapolationCheck(DevModel const& m, BatchView const& b, int sms, cu
 void launchNetworkFP64(DevModel const& m, BatchView const& b, int derivatives, int sms, cudaStream_t st)
 {
     // tiles of 32 atoms (16 for wide networks) while their shared memory leaves at least two blocks per SM
-    int d32 = 0, d16 = 0, t32 = 0, t16 = 0;
+    int d32 = 0, d16 = 0, d8 = 0, t32 = 0, t16 = 0, t8 = 0;
     for (int e = 0; e < m.numElements; ++e)
     {
         d32 = std::max(d32, netSmemDoubles(m.el[e], netRow<32>()));
         d16 = std::max(d16, netSmemDoubles(m.el[e], netRow<16>()));
+        d8 = std::max(d8, netSmemDoubles(m.el[e], netRow<8>()));
         t32 += (b.elemBegin[e + 1] - b.elemBegin[e] + 31) / 32;
         t16 += (b.elemBegin[e + 1] - b.elemBegin[e] + 15) / 16;
+        t8 += (b.elemBegin[e + 1] - b.elemBegin[e] + 7) / 8;
     }
     auto tiled = [&](auto kernel, size_t bytes, int tiles) {
         if (tiles == 0) return;
@@ -574,8 +602,13 @@ void launchNetworkFP64(DevModel const& m, BatchView const& b, int derivatives, i
         kernel<<<std::min(tiles, sms * perSM), kNetThreads, bytes, st>>>(m, b, derivatives);
     };
     constexpr size_t kTileBudget = 110 * 1024;
-    if ((size_t)d32 * sizeof(double) <= kTileBudget) return tiled(kNetworkTiled<32>, (size_t)d32 * sizeof(double), t32);
-    if ((size_t)d16 * sizeof(double) <= kTileBudget) return tiled(kNetworkTiled<16>, (size_t)d16 * sizeof(double), t16);
+    // Fewer tiles of 32 than SMs: tiles of 8 in units of 2 atoms, four times the blocks and a quarter
+    // of the serial activations per thread (192 atoms: 34 -> 18 us; 4,320 atoms: 39 -> 21 us; from one
+    // tile of 32 per SM on the wide units' fewer weight loads win).  Every sum keeps its order.
+    if (t32 < sms && (size_t)d8 * sizeof(double) <= kTileBudget)
+        return tiled(kNetworkTiled<8, 2>, (size_t)d8 * sizeof(double), t8);
+    if ((size_t)d32 * sizeof(double) <= kTileBudget) return tiled(kNetworkTiled<32, 8>, (size_t)d32 * sizeof(double), t32);
+    if ((size_t)d16 * sizeof(double) <= kTileBudget) return tiled(kNetworkTiled<16, 8>, (size_t)d16 * sizeof(double), t16);
     size_t smem = sizeof(NNWarpSmem) * kNNWarps;
     setDynamicSmemOnce(reinterpret_cast<const void*>(kNetworkFP64), smem);
     int blocks = (b.N + kNNWarps - 1) / kNNWarps;

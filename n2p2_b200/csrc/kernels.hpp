@@ -92,6 +92,7 @@ void cudaCheck(cudaError_t e, char const* what);
 void setDynamicSmemOnce(const void* kernel, size_t bytes);
 
 // neighbour list
+// Positions to internal units; also clears the status word and the cell counts.
 void launchPreparePositions(BatchView const& b, const double* rin, int doRemap, int doNormalize, double convLength,
                             cudaStream_t st);
 void launchNeighborBuild(BatchView const& b, double rc2, cudaStream_t st);
