@@ -224,6 +224,7 @@ struct DevModel
     const DevCompactFn*     compactFns;
     int compactRows;      // largest nR of a wide angular group
     int compactAngCore;   // the core of every angular part of the staged angular groups, or 0 if they differ
+    int compactRadCore;   // the same of every radial part of these groups
     int compactNarrowStaged;   // every narrow group fits the staged kernels (one grid chunk, a short walk)
     int compactCols;      // largest nA of a staged angular group
 };

@@ -395,7 +395,7 @@ void DeviceModel::upload(Model const& m)
     std::vector<DevCompactMember> compactMembers;
     std::vector<DevCompactFn> compactFns;
     int compactRows = 0;
-    int compactAngCore = -1;   // -1: no staged angular part seen yet
+    int compactAngCore = -1, compactRadCore = -1;   // -1: no staged angular group seen yet
     int compactNarrowStaged = 1;
     int compactCols = 0;
     std::vector<DevScaling> scaling;
@@ -684,6 +684,8 @@ void DeviceModel::upload(Model const& m)
                 {
                     compactRows = std::max(compactRows, cg.nR);
                     compactCols = std::max(compactCols, cg.nA);
+                    for (auto const& f : rad)
+                        compactRadCore = (compactRadCore == -1 || compactRadCore == f.core) ? f.core : 0;
                     for (auto const& f : ang)
                         compactAngCore = (compactAngCore == -1 || compactAngCore == f.core) ? f.core : 0;
                 }
@@ -789,6 +791,7 @@ void DeviceModel::upload(Model const& m)
     v.compactFns = compactFns_;
     v.compactRows = compactRows;
     v.compactAngCore = std::max(compactAngCore, 0);
+    v.compactRadCore = std::max(compactRadCore, 0);
     v.compactNarrowStaged = compactNarrowStaged;
     v.compactCols = compactCols;
     v.groups = groups_;

@@ -25,6 +25,7 @@
 //    neighbour) and its half of the self force.
 // No atomics; the same result on every run.
 #include <algorithm>
+#include <type_traits>
 
 #include "kernels.hpp"
 #include "kernels_common.cuh"
@@ -495,13 +496,23 @@ __global__ void __launch_bounds__(128, 2) kCompactForces(DevModel model, BatchVi
 // the G pass a batch is a k = 32 slice of the product S = P^T A, P the
 // pairs' radial products f_r f_r (32 x nR) and A their angular parts
 // (32 x nA), run on the FP64 tensor cores (mma m8n8k4, FP64 accumulation)
-// from a per-warp shared tile; the force pass adds a batch round by round to
+// from a per-warp shared tile, or, where the grid fits a lane's registers, kept
+// there (kCompactGridValues); the force pass adds a batch round by round to
 // the warp's own force array, so no slot is written twice at once.  Every
 // sum runs in a fixed order.
+// Bound: FP64 instructions and their latency at 12 warps per SM.  Branch-free
+// p2 parts, register grid, 16-byte (value, derivative) and weight loads: 16
+// Anisole boxes (4,096 atoms, 200 neighbours) G 2.36 -> 1.33 ms, forces 3.89
+// -> 2.88 ms; with one-warp blocks for molecules, 1,024 of them G 0.44 -> 0.22
+// ms and forces 0.91 -> 0.39 ms.
 constexpr int kWideRows = kCompactStageRows;   // radial parts per chunk
 constexpr int kWideCols = kCompactStageCols;   // angular parts per chunk
-constexpr int kWideCap = 256;   // staged neighbours; atoms with more run the direct kernels
-constexpr int kWideWarps = 4;
+// Two shapes of a block: four warps for atoms with up to kWideCap neighbours
+// (more run the direct kernels), one warp for those with up to kSmallCap
+// (molecules: a pair list of a few batches; 15 neighbours make 105 pairs, and
+// four warps per atom spent their time in barriers).
+constexpr int kWideCap = 256, kWideWarps = 4;
+constexpr int kSmallCap = 64, kSmallWarps = 1;
 constexpr int kCellStride = 8;  // G pass cell sums: row r, column a at r * 8 + a
 constexpr int kTileStride = 36; // per-warp tile: 32 pairs per row, padded against bank conflicts
 
@@ -516,29 +527,45 @@ __host__ __device__ constexpr int cellCount() { return tileRows<NARROW>() * kCel
 static_assert(kWideRows + kCompactImpure <= 16, "impure rows beyond the mma halves");
 static_assert(kWideCols <= kCellStride && kWideCols <= 8, "angular parts beyond the mma's 8 columns");
 
-// Value and derivative of a radial part at r (0 outside the open window):
-// CompactFunction::fdf with the part's core and asymmetry.
-__device__ __forceinline__ void compactPartFdf(DevCompactFn const& f, double x, double& v, double& dv)
+// A part in the form of partFdf: u = scale x + shift, |u| < 1 inside the window.
+struct alignas(16) PartScale
 {
-    v = 0.0;
-    dv = 0.0;
-    if (x > f.left && x < f.right) compactFdf(f.core, f.asym, f.center, f.scale, x, v, dv);
-}
+    double scale, shift;
+};
 
-// The same for an angular part (symmetric core), the core fixed at compile
-// time when ACORE != 0 (every angular part of the model has that core).
-template <int ACORE>
-__device__ __forceinline__ void angularPartFdf(DevCompactFn const& f, double x, double& v, double& dv)
+// Value and derivative of a part at x (0 outside its open window):
+// CompactFunction::fdf with the part's core and, for the radial ones, its
+// asymmetry.  CORE kCorePoly2 (every part of the model is p2): without a
+// branch and without the cancellation of the expanded polynomial at the
+// window's ends, with w = max(1 - |u|, 0),
+//   symmetric   f = w^3 (1 + 3x + 6x^2), x = |u|; f' = -30 x^2 w^2 sign(u) scale
+//   asymmetric  the same of y = (2 - x) x = 1 - w^2, times dy/dx = 2 w.
+template <int CORE, bool ANGULAR>
+__device__ __forceinline__ void partFdf(DevCompactFn const& f, PartScale const& p, double x, double& v, double& dv)
 {
-    v = 0.0;
-    dv = 0.0;
-    if (x > f.left && x < f.right)
+    if constexpr (CORE == kCorePoly2)
     {
-        const double u = (x - f.center) * f.scale;
-        double fx, dfx;
-        coreFdf(ACORE != 0 ? ACORE : f.core, fabs(u), fx, dfx);
-        v = fx;
-        dv = dfx * copysign(f.scale, u);
+        const double u = fma(x, p.scale, p.shift);
+        double w = 1.0 - fabs(u);
+        w = __double2hiint(w) < 0 ? 0.0 : w;
+        if (!ANGULAR && f.asym)
+        {
+            const double q = w * w, y = 1.0 - q, yq = y * q;
+            v = q * q * q * fma(fma(6.0, y, 3.0), y, 1.0);
+            dv = -60.0 * copysign(p.scale, u) * (yq * yq) * w;
+        }
+        else
+        {
+            const double a = fabs(u);
+            v = w * w * w * fma(fma(6.0, a, 3.0), a, 1.0);
+            dv = -30.0 * p.scale * (u * a) * (w * w);
+        }
+    }
+    else
+    {
+        v = 0.0;
+        dv = 0.0;
+        if (x > f.left && x < f.right) compactFdf(f.core, ANGULAR ? 0 : f.asym, f.center, f.scale, x, v, dv);
     }
 }
 
@@ -557,51 +584,60 @@ __device__ __forceinline__ void mmaF64(double& d0, double& d1, double a, double 
 // force pass's per-warp force arrays and cell weights.
 struct WideSmem
 {
-    double *x, *y, *z, *r, *rinv;   // [kWideCap]
-    double *rad, *drad;             // [rows][kWideCap] radial values (and derivatives, force pass)
-    double *h;                      // force pass: [warps][3][kWideCap]
-    double *tile;                   // G pass: [warps][tile rows + kWideCols][kTileStride]
-    double *cell;                   // G pass: [warps][tile rows * kCellStride] sums; force pass: W [kWideRows][kWideCols]
+    double *x, *y, *z, *r, *rinv;   // [CAP]
+    double *rad;                    // G pass: [rows][CAP] radial values, or slot-major (kRadPitch per slot)
+    double2 *radd;                  // force pass: [rows][CAP] radial values and derivatives
+    double *h;                      // force pass: [WARPS][3][CAP]
+    double *tile;                   // G pass: [WARPS][tile rows + kWideCols][kTileStride], or sums scratch
+    double *cell;                   // G pass: [WARPS][tile rows * kCellStride] sums; force pass: W [kWideRows][COLS]
     double *walkW;                  // force pass: [kCompactWalk] weights of the replayed impure members
-    DevCompactFn* fn;               // [kWideRows + kWideCols]: radial parts, then angular parts
+    PartScale* fs;                  // [kWideRows + kWideCols]: radial parts, then angular parts
+    DevCompactFn* fn;               // the same
     int* walk;                      // [kCompactWalk][4]: replayed members' rIdx, aIdx, calcComp, impure
     int* blockBegin;                // [kDevMaxElements + 1]
-    short* perm;                    // [kWideCap] slot -> position in the atom's list
-    unsigned char* el;              // [kWideCap]
+    short* perm;                    // [CAP] slot -> position in the atom's list
+    unsigned char* el;              // [CAP]
 };
 
-__host__ __device__ inline size_t wideDoubles(int rows, int warps, bool forces, bool narrow)
+constexpr int kRadPitch = 10;       // doubles per slot: 80 bytes, 16-byte loads of eight slots without conflicts
+
+template <int CAP, int WARPS>
+__host__ __device__ inline size_t wideDoubles(int rows, bool forces, bool narrow)
 {
     const size_t tile = narrow ? tileDoubles<true>() + cellCount<true>() : tileDoubles<false>() + cellCount<false>();
-    return 5 * kWideCap + (size_t)rows * kWideCap * (forces ? 2 : 1) +
-           (forces ? (size_t)warps * 3 * kWideCap + kWideRows * kWideCols + kCompactWalk : (size_t)warps * tile);
+    return 5 * CAP + 2 * (kWideRows + kWideCols) +
+           (forces ? (size_t)rows * CAP * 2 + (size_t)WARPS * 3 * CAP + kWideRows * kWideCols + kCompactWalk
+                   : (size_t)kRadPitch * CAP + (size_t)WARPS * tile);
 }
 
-__host__ __device__ inline size_t wideSmemBytes(int rows, int warps, bool forces, bool narrow)
+template <int CAP, int WARPS>
+__host__ __device__ inline size_t wideSmemBytes(int rows, bool forces, bool narrow)
 {
-    return wideDoubles(rows, warps, forces, narrow) * sizeof(double) + (kWideRows + kWideCols) * sizeof(DevCompactFn) +
-           (4 * kCompactWalk + kDevMaxElements + 1) * sizeof(int) + kWideCap * sizeof(short) + kWideCap;
+    return wideDoubles<CAP, WARPS>(rows, forces, narrow) * sizeof(double) + (kWideRows + kWideCols) * sizeof(DevCompactFn) +
+           (4 * kCompactWalk + kDevMaxElements + 1) * sizeof(int) + CAP * sizeof(short) + CAP;
 }
 
-__device__ __forceinline__ WideSmem wideCarve(char* base, int rows, int warps, bool forces, bool narrow)
+template <int CAP, int WARPS>
+__device__ __forceinline__ WideSmem wideCarve(char* base, int rows, bool forces, bool narrow)
 {
     WideSmem S;
     double* d = reinterpret_cast<double*>(base);
     S.x = d;
-    S.y = d + kWideCap;
-    S.z = d + 2 * kWideCap;
-    S.r = d + 3 * kWideCap;
-    S.rinv = d + 4 * kWideCap;
-    d += 5 * kWideCap;
-    S.rad = d;
-    d += rows * kWideCap;
-    S.drad = S.h = S.tile = S.walkW = nullptr;
+    S.y = d + CAP;
+    S.z = d + 2 * CAP;
+    S.r = d + 3 * CAP;
+    S.rinv = d + 4 * CAP;
+    d += 5 * CAP;
+    S.fs = reinterpret_cast<PartScale*>(d);
+    d += 2 * (kWideRows + kWideCols);
+    S.rad = S.h = S.tile = S.walkW = nullptr;
+    S.radd = nullptr;
     if (forces)
     {
-        S.drad = d;
-        d += rows * kWideCap;
+        S.radd = reinterpret_cast<double2*>(d);
+        d += (size_t)rows * CAP * 2;
         S.h = d;
-        d += warps * 3 * kWideCap;
+        d += WARPS * 3 * CAP;
         S.cell = d;
         d += kWideRows * kWideCols;
         S.walkW = d;
@@ -609,20 +645,84 @@ __device__ __forceinline__ WideSmem wideCarve(char* base, int rows, int warps, b
     }
     else
     {
+        S.rad = d;
+        d += kRadPitch * CAP;
         S.tile = d;
-        d += warps * (narrow ? tileDoubles<true>() : tileDoubles<false>());
+        d += WARPS * (narrow ? tileDoubles<true>() : tileDoubles<false>());
         S.cell = d;
-        d += warps * (narrow ? cellCount<true>() : cellCount<false>());
+        d += WARPS * (narrow ? cellCount<true>() : cellCount<false>());
     }
     S.fn = reinterpret_cast<DevCompactFn*>(d);
     S.walk = reinterpret_cast<int*>(S.fn + kWideRows + kWideCols);
     S.blockBegin = S.walk + 4 * kCompactWalk;
     S.perm = reinterpret_cast<short*>(S.blockBegin + kDevMaxElements + 1);
-    S.el = reinterpret_cast<unsigned char*>(S.perm + kWideCap);
+    S.el = reinterpret_cast<unsigned char*>(S.perm + CAP);
     return S;
 }
 
-// Stage the atom's n <= kWideCap neighbours sorted by element (stable).
+// Barrier of a block of WARPS warps.
+template <int WARPS>
+__device__ __forceinline__ void blockSync()
+{
+    if (WARPS == 1) __syncwarp();
+    else __syncthreads();
+}
+
+// The block's atoms: those of the type with lower < n <= CAP neighbours,
+// found blockDim.x at a time; f(i) runs on the whole block.
+template <int TYPE, int CAP, int WARPS, typename F>
+__device__ __forceinline__ void forTypeAtoms(DevModel const& model, BatchView const& b, int lower, F f)
+{
+    __shared__ unsigned todo[WARPS];
+    constexpr int T = WARPS * 32;
+    const int tid = threadIdx.x;
+    // consecutive atoms go to different blocks
+    for (int base = 0; base < b.N; base += (int)gridDim.x * T)
+    {
+        const int i = base + tid * (int)gridDim.x + (int)blockIdx.x;
+        bool mine = false;
+        if (i < b.N)
+        {
+            const int64_t off = b.nbrOffset[i], end = b.nbrOffset[i + 1];
+            const int n = (int)(end - off);
+            mine = end <= b.nbrCapacity && n > lower && n <= CAP;
+            if (mine)
+            {
+                DevElement const& E = model.el[b.elem[i]];
+                mine = false;
+                for (int g = 0; g < E.compactCount; ++g)
+                    mine = mine || model.compactGroups[E.compactBegin + g].type == TYPE;
+            }
+        }
+        const unsigned bal = __ballot_sync(kFullMask, mine);
+        if ((tid & 31) == 0) todo[tid >> 5] = bal;
+        blockSync<WARPS>();
+        for (int w = 0; w < WARPS; ++w)
+            for (unsigned m = todo[w]; m; m &= m - 1)
+                f(base + (w * 32 + __ffs(m) - 1) * (int)gridDim.x + (int)blockIdx.x);
+        blockSync<WARPS>();
+    }
+}
+
+// Sums of eight per-lane values over the warp in a fixed order: lane 4 c
+// returns the sum of v[c].  `scratch`: 8 x kTileStride doubles of the warp.
+__device__ __forceinline__ double eightSums(double const (&v)[8], double* scratch, int lane)
+{
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 8; ++c) scratch[c * kTileStride + lane] = v[c];
+    __syncwarp();
+    const double* p = scratch + (lane >> 2) * kTileStride + (lane & 3);
+    double s = p[0];
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += p[4 * k];
+    s += __shfl_xor_sync(kFullMask, s, 1);
+    s += __shfl_xor_sync(kFullMask, s, 2);
+    return s;
+}
+
+// Stage the atom's neighbours sorted by element (stable).
+template <int WARPS>
 __device__ void wideStage(WideSmem const& S, DevModel const& model, BatchView const& b, int64_t off, int n, int tid,
                           int threads)
 {
@@ -661,7 +761,7 @@ __device__ void wideStage(WideSmem const& S, DevModel const& model, BatchView co
             }
         }
     }
-    __syncthreads();
+    blockSync<WARPS>();
     for (int s = tid; s < n; s += threads)
     {
         const int64_t e = off + S.perm[s];
@@ -673,7 +773,7 @@ __device__ void wideStage(WideSmem const& S, DevModel const& model, BatchView co
         S.rinv[s] = 1.0 / d;
         S.el[s] = b.nbrElem[e];
     }
-    __syncthreads();
+    blockSync<WARPS>();
 }
 
 // A group's pairs: the neighbours of its element pair (all neighbours for the
@@ -713,36 +813,48 @@ __device__ __forceinline__ WidePairs widePairs(WideSmem const& S, DevCompactGrou
 
 // Parts of the chunk (rows r0.., columns a0..), the radial values of the
 // group's slots and, for a narrow group, its replayed members.
-template <bool FORCES, bool NARROW>
+template <bool FORCES, bool NARROW, int CORE, int CAP, int WARPS, bool SLOTMAJOR>
 __device__ __forceinline__ void wideStageChunk(WideSmem const& S, DevModel const& model, DevCompactGroup const& G,
                                                WidePairs const& P, const DevCompactMember* mem, const double* dEdG,
-                                               DevElement const& E, int r0, int nRc, int a0, int nAc, int tid,
-                                               int threads)
+                                               DevElement const& E, int r0, int nRc, int a0, int nAc, int tid)
 {
-    if (tid < nRc) S.fn[tid] = model.compactFns[G.fnBegin + r0 + tid];
-    else if (tid >= kWideRows && tid < kWideRows + nAc)
-        S.fn[tid] = model.compactFns[G.fnBegin + G.nR + a0 + tid - kWideRows];
-    if (NARROW && tid >= 32 && tid < 32 + G.walkEnd - G.walkBegin)
+    constexpr int threads = WARPS * 32;
+    if (tid < kWideRows + kWideCols)
     {
-        const int st = tid - 32;
-        DevCompactMember const& M = mem[G.walkBegin + st];
-        S.walk[4 * st] = M.rIdx;
-        S.walk[4 * st + 1] = M.aIdx;
-        S.walk[4 * st + 2] = M.calcComp;
-        S.walk[4 * st + 3] = M.impure;
-        if (FORCES)
-            S.walkW[st] = M.impure >= 0 ? dEdG[M.sf] * model.scaling[E.sfBegin + M.sf].scalingFactor : 0.0;
+        const bool radial = tid < kWideRows;
+        const int q = radial ? tid : tid - kWideRows;
+        PartScale p{0.0, 2.0};   // an absent part: outside everywhere
+        if (q < (radial ? nRc : nAc))
+        {
+            const DevCompactFn f = model.compactFns[G.fnBegin + (radial ? r0 + q : G.nR + a0 + q)];
+            S.fn[tid] = f;
+            p.scale = f.scale;
+            p.shift = -f.center * f.scale;
+        }
+        S.fs[tid] = p;
     }
-    __syncthreads();
-    for (int k = tid; k < nRc * P.ns; k += threads)
+    if (NARROW)
+        for (int st = tid; st < G.walkEnd - G.walkBegin; st += threads)
+        {
+            DevCompactMember const& M = mem[G.walkBegin + st];
+            S.walk[4 * st] = M.rIdx;
+            S.walk[4 * st + 1] = M.aIdx;
+            S.walk[4 * st + 2] = M.calcComp;
+            S.walk[4 * st + 3] = M.impure;
+            if (FORCES)
+                S.walkW[st] = M.impure >= 0 ? dEdG[M.sf] * model.scaling[E.sfBegin + M.sf].scalingFactor : 0.0;
+        }
+    blockSync<WARPS>();
+    const int rows = SLOTMAJOR ? kRadPitch : nRc;
+    for (int k = tid; k < rows * P.ns; k += threads)
     {
         const int rr = k / P.ns;
         const int j = k - rr * P.ns;
         const int s = j < P.nA ? P.A0 + j : P.B0 + (j - P.nA);
-        double f, df;
-        compactPartFdf(S.fn[rr], S.r[s], f, df);
-        S.rad[rr * kWideCap + s] = f;
-        if (FORCES) S.drad[rr * kWideCap + s] = df;
+        double f = 0.0, df = 0.0;
+        if (!SLOTMAJOR || rr < nRc) partFdf<CORE, false>(S.fn[rr], S.fs[rr], S.r[s], f, df);
+        if (FORCES) S.radd[rr * CAP + s] = make_double2(f, df);
+        else S.rad[SLOTMAJOR ? s * kRadPitch + rr : rr * CAP + s] = f;
     }
 }
 
@@ -750,6 +862,7 @@ __device__ __forceinline__ void wideStageChunk(WideSmem const& S, DevModel const
 // bit r (r < 32) when the first neighbour's radial part r is not 0 and the
 // second neighbour's distance and r_jk are inside its window; bit 32 + a when
 // the angle is inside angular part a's window.
+template <bool FORCES, int CAP>
 __device__ __forceinline__ unsigned long long walkMasks(WideSmem const& S, int u, int v, double rjk, double acost,
                                                        int nRc, int nAc)
 {
@@ -760,7 +873,7 @@ __device__ __forceinline__ unsigned long long walkMasks(WideSmem const& S, int u
     for (int r = 0; r < nRc; ++r)
     {
         DevCompactFn const& f = S.fn[r];
-        const double r1 = S.rad[r * kWideCap + s1];
+        const double r1 = FORCES ? S.radd[r * CAP + s1].x : S.rad[r * CAP + s1];
         if (r1 != 0.0 && rsec > f.left && rsec < f.right && rjk > f.left && rjk < f.right)
             mR |= 1u << r;
     }
@@ -772,57 +885,46 @@ __device__ __forceinline__ unsigned long long walkMasks(WideSmem const& S, int u
     return ((unsigned long long)mA << 32) | mR;
 }
 
-template <int TYPE>
-__device__ __forceinline__ bool hasType(DevModel const& model, DevElement const& E)
-{
-    for (int g = 0; g < E.compactCount; ++g)
-        if (model.compactGroups[E.compactBegin + g].type == TYPE) return true;
-    return false;
-}
-
-template <int TYPE, int ACORE>
-__global__ void __launch_bounds__(kWideWarps * 32, 4) kCompactWideValues(DevModel model, BatchView b, int rows)
+template <int TYPE, int CORE, int CAP, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
+    kCompactWideValues(const __grid_constant__ DevModel model, const __grid_constant__ BatchView b, int rows, int lower)
 {
     constexpr bool WEIGHTED = TYPE >= 24;
     constexpr bool NARROW = TYPE == 21 || TYPE == 24;
-    constexpr int T = kWideWarps * 32;
+    constexpr int T = WARPS * 32;
     constexpr int TR = tileRows<NARROW>();
     extern __shared__ __align__(16) char smemRaw[];
-    const WideSmem S = wideCarve(smemRaw, rows, kWideWarps, false, NARROW);
+    const WideSmem S = wideCarve<CAP, WARPS>(smemRaw, rows, false, NARROW);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double* PT = S.tile + warp * tileDoubles<NARROW>();   // this warp's tile: radial products, then angular parts
     double* AT = PT + TR * kTileStride;
     double* cw = S.cell + warp * cellCount<NARROW>();
     const int g4 = lane >> 2, t4 = lane & 3;              // mma fragment row / column of the lane
-    for (int i = blockIdx.x; i < b.N; i += gridDim.x)
-    {
+    forTypeAtoms<TYPE, CAP, WARPS>(model, b, lower, [&](int i) {
         DevElement const& E = model.el[b.elem[i]];
-        if (!hasType<TYPE>(model, E)) continue;
         const int64_t off = b.nbrOffset[i];
-        const int64_t end = b.nbrOffset[i + 1];
-        const int n = (int)(end - off);
-        if (end > b.nbrCapacity || n > kWideCap) continue;
-        wideStage(S, model, b, off, n, tid, T);
+        const int n = (int)(b.nbrOffset[i + 1] - off);
+        wideStage<WARPS>(S, model, b, off, n, tid, T);
         for (int g = 0; g < E.compactCount; ++g)
         {
             DevCompactGroup const G = model.compactGroups[E.compactBegin + g];
             if (G.type != TYPE) continue;
             const WidePairs P = widePairs<WEIGHTED>(S, G, n);
             const DevCompactMember* mem = model.compactMembers + G.memberBegin;
-            const int q = (32 * kWideWarps) / P.ph.minor, rem = 32 * kWideWarps - q * P.ph.minor;
+            const int q = (32 * WARPS) / P.ph.minor, rem = 32 * WARPS - q * P.ph.minor;
             const int nImp = NARROW ? G.numImpure : 0;
             const int wl = NARROW ? G.walkEnd - G.walkBegin : 0;
             for (int r0 = 0; r0 < G.nR; r0 += kWideRows)
                 for (int a0 = 0; a0 < G.nA; a0 += kWideCols)
                 {
                     const int nRc = min(kWideRows, G.nR - r0), nAc = min(kWideCols, G.nA - a0);
-                    wideStageChunk<false, NARROW>(S, model, G, P, mem, nullptr, E, r0, nRc, a0, nAc, tid, T);
-                    __syncthreads();
+                    wideStageChunk<false, NARROW, CORE, CAP, WARPS, false>(S, model, G, P, mem, nullptr, E, r0, nRc, a0, nAc, tid);
+                    blockSync<WARPS>();
                     // sums of tile rows 0-7 (c0x) and 8-15 (c1x), columns 2 t4 + {0, 1}
                     double c00 = 0.0, c01 = 0.0, c10 = 0.0, c11 = 0.0;
                     Cursor cur;
                     cur.init(P.ph, 32 * warp + lane);
-                    for (int p0 = 32 * warp; p0 < P.ph.count; p0 += 32 * kWideWarps, cur.advance(P.ph, q, rem))
+                    for (int p0 = 32 * warp; p0 < P.ph.count; p0 += 32 * WARPS, cur.advance(P.ph, q, rem))
                     {
                         int u = 0, v = 0;
                         bool ok = p0 + lane < P.ph.count && cur.slots(P.ph, u, v);
@@ -850,16 +952,16 @@ __global__ void __launch_bounds__(kWideWarps * 32, 4) kCompactWideValues(DevMode
                             for (int a = 0; a < nAc; ++a)
                             {
                                 double f, df;
-                                angularPartFdf<ACORE>(S.fn[kWideRows + a], acost, f, df);
+                                partFdf<CORE, true>(S.fn[kWideRows + a], S.fs[kWideRows + a], acost, f, df);
                                 AT[a * kTileStride + lane] = WEIGHTED ? f * zw : f;
                             }
                             for (int r = 0; r < nRc; ++r)
                             {
-                                double pr = S.rad[r * kWideCap + u] * S.rad[r * kWideCap + v];
+                                double pr = S.rad[r * CAP + u] * S.rad[r * CAP + v];
                                 if (NARROW)
                                 {
                                     double fq, dfq;
-                                    compactPartFdf(S.fn[r], rjk, fq, dfq);
+                                    partFdf<CORE, false>(S.fn[r], S.fs[r], rjk, fq, dfq);
                                     pr *= fq;
                                 }
                                 PT[r * kTileStride + lane] = pr;
@@ -867,7 +969,7 @@ __global__ void __launch_bounds__(kWideWarps * 32, 4) kCompactWideValues(DevMode
                             if (NARROW && wl > 0)
                             {
                                 // replay the carried j-k radial part for the impure members (their own rows)
-                                const unsigned long long mk = walkMasks(S, u, v, rjk, acost, nRc, nAc);
+                                const unsigned long long mk = walkMasks<false, CAP>(S, u, v, rjk, acost, nRc, nAc);
                                 int src = -1;
                                 bool cskip = false;
                                 double qs = 0.0;
@@ -884,7 +986,7 @@ __global__ void __launch_bounds__(kWideWarps * 32, 4) kCompactWideValues(DevMode
                                         if (R != src)
                                         {
                                             double dq;
-                                            compactPartFdf(S.fn[R], rjk, qs, dq);
+                                            partFdf<CORE, false>(S.fn[R], S.fs[R], rjk, qs, dq);
                                             src = R;
                                         }
                                         cskip = false;
@@ -892,7 +994,7 @@ __global__ void __launch_bounds__(kWideWarps * 32, 4) kCompactWideValues(DevMode
                                     const int imp = S.walk[4 * st + 3];
                                     if (imp >= 0)
                                         PT[(kWideRows + imp) * kTileStride + lane] =
-                                            S.rad[R * kWideCap + u] * S.rad[R * kWideCap + v] * qs;
+                                            S.rad[R * CAP + u] * S.rad[R * CAP + v] * qs;
                                 }
                             }
                         }
@@ -926,7 +1028,7 @@ __global__ void __launch_bounds__(kWideWarps * 32, 4) kCompactWideValues(DevMode
                         cw[(g4 + 8) * kCellStride + 2 * t4] = c10;
                         cw[(g4 + 8) * kCellStride + 2 * t4 + 1] = c11;
                     }
-                    __syncthreads();
+                    blockSync<WARPS>();
                     for (int mi = tid; mi < G.memberCount; mi += T)
                     {
                         DevCompactMember const& M = mem[mi];
@@ -935,70 +1037,166 @@ __global__ void __launch_bounds__(kWideWarps * 32, 4) kCompactWideValues(DevMode
                         // impure members (narrow groups) have rows of their own after the grid's
                         const int c = ((NARROW && M.impure >= 0) ? kWideRows + M.impure : rr) * kCellStride + aa;
                         double sum = S.cell[c];
-                        for (int w = 1; w < kWideWarps; ++w) sum += S.cell[w * cellCount<NARROW>() + c];
+                        for (int w = 1; w < WARPS; ++w) sum += S.cell[w * cellCount<NARROW>() + c];
                         b.G[(size_t)i * b.gStride + M.sf] = scaleG(model.scaling[E.sfBegin + M.sf], sum);
                     }
-                    __syncthreads();
+                    blockSync<WARPS>();
                 }
         }
-    }
+    });
 }
 
-template <int TYPE, int ACORE, int COLS>
-__global__ void __launch_bounds__(kWideWarps * 32, 3) kCompactWideForces(DevModel model, BatchView b, int rows)
+// G pass of the wide types without a narrow window where the grid fits
+// kGridRows x kGridCols registers per lane and every part is p2: the sums
+// S[r][a] stay in each lane's registers over the atom's pairs (54 fused
+// multiply-adds per pair of a 9 x 6 grid), instead of a shared tile per 32
+// pairs whose product on the FP64 tensor cores (16 x 8 for 9 x 6 cells) costs
+// more pipe time than the plain FMAs and two shared passes.
+constexpr int kGridRows = 10, kGridCols = 6;
+
+template <int TYPE, int ROWS, int CAP, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
+    kCompactGridValues(const __grid_constant__ DevModel model, const __grid_constant__ BatchView b, int rows, int lower)
+{
+    constexpr bool WEIGHTED = TYPE >= 24;
+    constexpr int T = WARPS * 32, CELLS = ROWS * kGridCols;
+    extern __shared__ __align__(16) char smemRaw[];
+    const WideSmem S = wideCarve<CAP, WARPS>(smemRaw, rows, false, false);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double* scratch = S.tile + warp * tileDoubles<false>();
+    double* cw = S.cell + warp * cellCount<false>();
+    forTypeAtoms<TYPE, CAP, WARPS>(model, b, lower, [&](int i) {
+        DevElement const& E = model.el[b.elem[i]];
+        const int64_t off = b.nbrOffset[i];
+        const int n = (int)(b.nbrOffset[i + 1] - off);
+        wideStage<WARPS>(S, model, b, off, n, tid, T);
+        for (int g = 0; g < E.compactCount; ++g)
+        {
+            DevCompactGroup const& G = model.compactGroups[E.compactBegin + g];
+            if (G.type != TYPE) continue;
+            const WidePairs P = widePairs<WEIGHTED>(S, G, n);
+            const DevCompactMember* mem = model.compactMembers + G.memberBegin;
+            const int q = (32 * WARPS) / P.ph.minor, rem = 32 * WARPS - q * P.ph.minor;
+            wideStageChunk<false, false, kCorePoly2, CAP, WARPS, true>(S, model, G, P, mem, nullptr, E, 0, G.nR, 0, G.nA, tid);
+            blockSync<WARPS>();
+            double acc[ROWS][kGridCols];
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r)
+#pragma unroll
+                for (int a = 0; a < kGridCols; ++a) acc[r][a] = 0.0;
+            Cursor cur;
+            cur.init(P.ph, 32 * warp + lane);
+            for (int p = 32 * warp + lane; p < P.ph.count; p += 32 * WARPS, cur.advance(P.ph, q, rem))
+            {
+                int u = 0, v = 0;
+                if (!cur.slots(P.ph, u, v)) continue;
+                const double cost = (S.x[u] * S.x[v] + S.y[u] * S.y[v] + S.z[u] * S.z[v]) * (S.rinv[u] * S.rinv[v]);
+                if (!(cost > -1.0 && cost < 1.0)) continue;
+                const double acost = acos(cost);
+                const double zw = WEIGHTED ? model.atomicNumber[S.el[u]] * model.atomicNumber[S.el[v]] : 1.0;
+                double ang[kGridCols];
+#pragma unroll
+                for (int a = 0; a < kGridCols; ++a)
+                {
+                    double df;
+                    partFdf<kCorePoly2, true>(S.fn[kWideRows + a], S.fs[kWideRows + a], acost, ang[a], df);
+                    if (WEIGHTED) ang[a] *= zw;
+                }
+                const double2* pu = reinterpret_cast<const double2*>(S.rad + u * kRadPitch);
+                const double2* pv = reinterpret_cast<const double2*>(S.rad + v * kRadPitch);
+#pragma unroll
+                for (int r = 0; r < ROWS; r += 2)
+                {
+                    const double2 fu = pu[r >> 1], fv = pv[r >> 1];
+                    const double p0 = fu.x * fv.x;
+#pragma unroll
+                    for (int a = 0; a < kGridCols; ++a) acc[r][a] += p0 * ang[a];
+                    if (r + 1 < ROWS)
+                    {
+                        const double p1 = fu.y * fv.y;
+#pragma unroll
+                        for (int a = 0; a < kGridCols; ++a) acc[r + 1][a] += p1 * ang[a];
+                    }
+                }
+            }
+            __syncwarp();
+#pragma unroll
+            for (int c0 = 0; c0 < CELLS; c0 += 8)
+            {
+                double v[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    v[k] = c0 + k < CELLS ? acc[(c0 + k < CELLS ? c0 + k : 0) / kGridCols][(c0 + k < CELLS ? c0 + k : 0) % kGridCols] : 0.0;
+                const double sum = eightSums(v, scratch, lane);
+                const int c = c0 + (lane >> 2);
+                if ((lane & 3) == 0 && c < CELLS) cw[c / kGridCols * kCellStride + c % kGridCols] = sum;
+            }
+            blockSync<WARPS>();
+            for (int mi = tid; mi < G.memberCount; mi += T)
+            {
+                DevCompactMember const& M = mem[mi];
+                const int c = M.rIdx * kCellStride + M.aIdx;
+                double sum = S.cell[c];
+                for (int w = 1; w < WARPS; ++w) sum += S.cell[w * cellCount<false>() + c];
+                b.G[(size_t)i * b.gStride + M.sf] = scaleG(model.scaling[E.sfBegin + M.sf], sum);
+            }
+            blockSync<WARPS>();
+        }
+    });
+}
+
+template <int TYPE, int CORE, int COLS, int CAP, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
+    kCompactWideForces(const __grid_constant__ DevModel model, const __grid_constant__ BatchView b, int rows, int lower)
 {
     constexpr bool WEIGHTED = TYPE >= 24;
     constexpr bool NARROW = TYPE == 21 || TYPE == 24;
-    constexpr int T = kWideWarps * 32;
-    static_assert(COLS <= kWideCols, "angular parts per chunk");
+    constexpr int T = WARPS * 32;
+    static_assert(COLS <= kWideCols && COLS % 2 == 0, "angular parts per chunk");
     extern __shared__ __align__(16) char smemRaw[];
-    const WideSmem S = wideCarve(smemRaw, rows, kWideWarps, true, NARROW);
+    const WideSmem S = wideCarve<CAP, WARPS>(smemRaw, rows, true, NARROW);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double* hw = S.h + warp * 3 * kWideCap;   // this warp's force array
-    for (int k = tid; k < kWideWarps * 3 * kWideCap; k += T) S.h[k] = 0.0;
-    for (int i = blockIdx.x; i < b.N; i += gridDim.x)
-    {
+    double* hw = S.h + warp * 3 * CAP;   // this warp's force array
+    for (int k = tid; k < WARPS * 3 * CAP; k += T) S.h[k] = 0.0;
+    forTypeAtoms<TYPE, CAP, WARPS>(model, b, lower, [&](int i) {
         DevElement const& E = model.el[b.elem[i]];
-        if (!hasType<TYPE>(model, E)) continue;
         const int64_t off = b.nbrOffset[i];
-        const int64_t end = b.nbrOffset[i + 1];
-        const int n = (int)(end - off);
-        if (end > b.nbrCapacity || n > kWideCap) continue;
+        const int n = (int)(b.nbrOffset[i + 1] - off);
         const double* dEdG = b.dEdG + (size_t)i * b.gStride;
-        wideStage(S, model, b, off, n, tid, T);
+        wideStage<WARPS>(S, model, b, off, n, tid, T);
         for (int g = 0; g < E.compactCount; ++g)
         {
-            DevCompactGroup const G = model.compactGroups[E.compactBegin + g];
+            DevCompactGroup const& G = model.compactGroups[E.compactBegin + g];
             if (G.type != TYPE) continue;
             const WidePairs P = widePairs<WEIGHTED>(S, G, n);
             if (P.ph.count == 0) continue;
             const DevCompactMember* mem = model.compactMembers + G.memberBegin;
-            const int q = (32 * kWideWarps) / P.ph.minor, rem = 32 * kWideWarps - q * P.ph.minor;
+            const int q = (32 * WARPS) / P.ph.minor, rem = 32 * WARPS - q * P.ph.minor;
             const int wl = NARROW ? G.walkEnd - G.walkBegin : 0;
             for (int r0 = 0; r0 < G.nR; r0 += kWideRows)
                 for (int a0 = 0; a0 < G.nA; a0 += COLS)
                 {
                     const int nRc = min(kWideRows, G.nR - r0), nAc = min(COLS, G.nA - a0);
-                    wideStageChunk<true, NARROW>(S, model, G, P, mem, dEdG, E, r0, nRc, a0, nAc, tid, T);
+                    wideStageChunk<true, NARROW, CORE, CAP, WARPS, false>(S, model, G, P, mem, dEdG, E, r0, nRc, a0, nAc, tid);
                     // cell weights of the grid's members (the impure ones are replayed per pair), summed
                     // in member order
-                    if (tid < kWideRows * COLS)
+                    for (int c = tid; c < kWideRows * COLS; c += T)
                     {
                         double w = 0.0;
                         for (int mi = 0; mi < G.memberCount; ++mi)
                         {
                             DevCompactMember const& M = mem[mi];
                             const int rr = M.rIdx - r0, aa = M.aIdx - a0;
-                            if (rr < 0 || rr >= nRc || aa < 0 || aa >= nAc || rr * COLS + aa != tid) continue;
+                            if (rr < 0 || rr >= nRc || aa < 0 || aa >= nAc || rr * COLS + aa != c) continue;
                             if (NARROW && M.impure >= 0) continue;
                             w += dEdG[M.sf] * model.scaling[E.sfBegin + M.sf].scalingFactor;
                         }
-                        S.cell[tid] = w;
+                        S.cell[c] = w;
                     }
-                    __syncthreads();
+                    blockSync<WARPS>();
                     Cursor cur;
                     cur.init(P.ph, 32 * warp + lane);
-                    for (int p0 = 32 * warp; p0 < P.ph.count; p0 += 32 * kWideWarps, cur.advance(P.ph, q, rem))
+                    for (int p0 = 32 * warp; p0 < P.ph.count; p0 += 32 * WARPS, cur.advance(P.ph, q, rem))
                     {
                         int u = 0, v = 0;
                         bool ok = p0 + lane < P.ph.count && cur.slots(P.ph, u, v);
@@ -1019,14 +1217,15 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) kCompactWideForces(DevMode
                             if (ok)
                             {
                                 const double acost = acos(cost);
-                                const double dacost = -1.0 / sqrt(1.0 - cost * cost);
+                                const double dacost = -rsqrt(fma(-cost, cost, 1.0));
                                 double ang[COLS], dang[COLS];
 #pragma unroll
                                 for (int a = 0; a < COLS; ++a)
                                 {
                                     ang[a] = 0.0;
                                     dang[a] = 0.0;
-                                    if (a < nAc) angularPartFdf<ACORE>(S.fn[kWideRows + a], acost, ang[a], dang[a]);
+                                    if (CORE == kCorePoly2 || a < nAc)
+                                        partFdf<CORE, true>(S.fn[kWideRows + a], S.fs[kWideRows + a], acost, ang[a], dang[a]);
                                 }
                                 // the reference's first neighbour of the pair is the lower list index
                                 const bool firstU = S.perm[u] < S.perm[v];
@@ -1036,25 +1235,30 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) kCompactWideForces(DevMode
                                 {
                                     if (r < nRc)
                                     {
-                                        const double ru = S.rad[r * kWideCap + u], rv = S.rad[r * kWideCap + v];
-                                        double dru = S.drad[r * kWideCap + u], drv = S.drad[r * kWideCap + v];
-                                        if (firstU ? ru == 0.0 : rv == 0.0)
+                                        const double2 fu = S.radd[r * CAP + u], fv = S.radd[r * CAP + v];
+                                        const double ru = fu.x, rv = fv.x;
+                                        double dru = fu.y, drv = fv.y;
+                                        // (the p2 form is 0 only where its derivative is)
+                                        if (CORE != kCorePoly2 && (firstU ? ru == 0.0 : rv == 0.0))
                                         {
                                             if (firstU) dru = 0.0;
                                             else drv = 0.0;
                                         }
                                         double U = 0.0, V = 0.0;
+                                        const double2* w2 = reinterpret_cast<const double2*>(S.cell + r * COLS);
 #pragma unroll
-                                        for (int a = 0; a < COLS; ++a)
+                                        for (int a = 0; a < COLS; a += 2)
                                         {
-                                            const double w = S.cell[r * COLS + a];
-                                            U += w * ang[a];
-                                            V += w * dang[a];
+                                            const double2 w = w2[a >> 1];
+                                            U += w.x * ang[a];
+                                            V += w.x * dang[a];
+                                            U += w.y * ang[a + 1];
+                                            V += w.y * dang[a + 1];
                                         }
                                         if (NARROW)
                                         {
                                             double fq, dfq;
-                                            compactPartFdf(S.fn[r], rjk, fq, dfq);
+                                            partFdf<CORE, false>(S.fn[r], S.fs[r], rjk, fq, dfq);
                                             Bu += dru * rv * fq * U;
                                             Bv += ru * drv * fq * U;
                                             Bjk += ru * rv * dfq * U;
@@ -1071,7 +1275,7 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) kCompactWideForces(DevMode
                                 if (NARROW && wl > 0)
                                 {
                                     // the impure members with the carried j-k radial part
-                                    const unsigned long long mk = walkMasks(S, u, v, rjk, acost, nRc, nAc);
+                                    const unsigned long long mk = walkMasks<true, CAP>(S, u, v, rjk, acost, nRc, nAc);
                                     int src = -1;
                                     bool cskip = false;
                                     double qs = 0.0, dqs = 0.0;
@@ -1087,17 +1291,17 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) kCompactWideForces(DevMode
                                         {
                                             if (R != src)
                                             {
-                                                compactPartFdf(S.fn[R], rjk, qs, dqs);
+                                                partFdf<CORE, false>(S.fn[R], S.fs[R], rjk, qs, dqs);
                                                 src = R;
                                             }
                                             cskip = false;
                                         }
                                         if (S.walk[4 * st + 3] < 0) continue;
                                         const double w = S.walkW[st];
-                                        const double ru = S.rad[R * kWideCap + u], rv = S.rad[R * kWideCap + v];
-                                        const double dru = S.drad[R * kWideCap + u], drv = S.drad[R * kWideCap + v];
+                                        const double2 fu = S.radd[R * CAP + u], fv = S.radd[R * CAP + v];
+                                        const double ru = fu.x, rv = fv.x, dru = fu.y, drv = fv.y;
                                         double fa, dfa;
-                                        angularPartFdf<ACORE>(S.fn[kWideRows + Ai], acost, fa, dfa);
+                                        partFdf<CORE, true>(S.fn[kWideRows + Ai], S.fs[kWideRows + Ai], acost, fa, dfa);
                                         Bu += w * (dru * rv * qs * fa);
                                         Bv += w * (ru * drv * qs * fa);
                                         Bjk += w * (ru * rv * dqs * fa);
@@ -1132,16 +1336,16 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) kCompactWideForces(DevMode
                                 const double xu = S.x[u], yu = S.y[u], zu = S.z[u];
                                 const double xv = S.x[v], yv = S.y[v], zv = S.z[v];
                                 hw[u] += cu * xu + gm * xv;
-                                hw[kWideCap + u] += cu * yu + gm * yv;
-                                hw[2 * kWideCap + u] += cu * zu + gm * zv;
+                                hw[CAP + u] += cu * yu + gm * yv;
+                                hw[2 * CAP + u] += cu * zu + gm * zv;
                                 hw[v] += cv * xv + gm * xu;
-                                hw[kWideCap + v] += cv * yv + gm * yu;
-                                hw[2 * kWideCap + v] += cv * zv + gm * zu;
+                                hw[CAP + v] += cv * yv + gm * yu;
+                                hw[2 * CAP + v] += cv * zv + gm * zu;
                             }
                             __syncwarp();
                         }
                     }
-                    __syncthreads();
+                    blockSync<WARPS>();
                 }
         }
         // per-entry forces (warp arrays summed in order) and the centre's share
@@ -1153,10 +1357,10 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) kCompactWideForces(DevMode
             for (int c = 0; c < 3; ++c)
             {
                 f[c] = 0.0;
-                for (int w = 0; w < kWideWarps; ++w)
+                for (int w = 0; w < WARPS; ++w)
                 {
-                    f[c] += S.h[(w * 3 + c) * kWideCap + s];
-                    S.h[(w * 3 + c) * kWideCap + s] = 0.0;
+                    f[c] += S.h[(w * 3 + c) * CAP + s];
+                    S.h[(w * 3 + c) * CAP + s] = 0.0;
                 }
             }
             if (f[0] != 0.0 || f[1] != 0.0 || f[2] != 0.0)
@@ -1179,17 +1383,17 @@ __global__ void __launch_bounds__(kWideWarps * 32, 3) kCompactWideForces(DevMode
             S.cell[3 * warp + 1] = sy;
             S.cell[3 * warp + 2] = sz;
         }
-        __syncthreads();
+        blockSync<WARPS>();
         if (tid == 0)
         {
             double t[3] = {0.0, 0.0, 0.0};
-            for (int w = 0; w < kWideWarps; ++w)
+            for (int w = 0; w < WARPS; ++w)
                 for (int c = 0; c < 3; ++c) t[c] += S.cell[3 * w + c];
             if (t[0] != 0.0 || t[1] != 0.0 || t[2] != 0.0)
                 for (int c = 0; c < 3; ++c) b.fSelf[3 * (size_t)i + c] += t[c];
         }
-        __syncthreads();
-    }
+        blockSync<WARPS>();
+    });
 }
 
 } // namespace
@@ -1202,12 +1406,6 @@ int compactBlocks(BatchView const& b, int sms)
     if (blocks < 1) blocks = 1;
     if (blocks > sms * 16) blocks = sms * 16;
     return blocks;
-}
-
-// One block per atom, at most perSM resident blocks per SM.
-int wideBlocks(BatchView const& b, int sms, int perSM)
-{
-    return std::max(1, std::min(b.N, sms * perSM));
 }
 
 } // namespace
@@ -1227,34 +1425,66 @@ int launchAngular(DevModel const& m, BatchView const& b, int sms, cudaStream_t s
         return 1;
     }
     const int rows = std::max(1, std::min(m.compactRows, kWideRows));
-    const size_t smem = wideSmemBytes(rows, kWideWarps, FORCES, NARROW);
-    auto staged = [&](auto kernel, int perSM) {
-        // resident blocks: the launch bound, or fewer when the stage is larger (228 KB of shared
-        // memory per SM, 1 KB of it reserved per block)
+    // resident blocks: the launch bound, or fewer when the stage is larger (228 KB of shared memory
+    // per SM, 1 KB of it reserved per block)
+    auto staged = [&](auto kernel, size_t smem, int warps, int perSM, int lower) {
         perSM = std::max(1, std::min(perSM, (int)(233472 / (smem + 1024))));
         setDynamicSmemOnce(reinterpret_cast<const void*>(kernel), smem);
-        kernel<<<wideBlocks(b, sms, perSM), kWideWarps * 32, smem, st>>>(m, b, rows);
+        kernel<<<std::max(1, std::min(b.N, sms * perSM)), warps * 32, smem, st>>>(m, b, rows, lower);
     };
-    const bool poly2 = m.compactAngCore == kCorePoly2;
-    if (FORCES)
+    const size_t large = wideSmemBytes<kWideCap, kWideWarps>(rows, FORCES, NARROW);
+    const size_t small = wideSmemBytes<kSmallCap, kSmallWarps>(rows, FORCES, NARROW);
+    const bool poly2 = m.compactAngCore == kCorePoly2 && m.compactRadCore == kCorePoly2;
+    if constexpr (FORCES)
     {
         // six angular parts per chunk where the model has no more (the SCAN and QM9 groups)
+        auto both = [&](auto core, auto cols) {
+            constexpr int C = decltype(core)::value, A = decltype(cols)::value;
+            staged(kCompactWideForces<TYPE, C, A, kSmallCap, kSmallWarps>, small, kSmallWarps, 12, -1);
+            staged(kCompactWideForces<TYPE, C, A, kWideCap, kWideWarps>, large, kWideWarps, 3, kSmallCap);
+        };
+        using Poly2 = std::integral_constant<int, kCorePoly2>;
+        using Any = std::integral_constant<int, 0>;
+        using Six = std::integral_constant<int, 6>;
+        using All = std::integral_constant<int, kWideCols>;
         if (m.compactCols <= 6)
         {
-            if (poly2) staged(kCompactWideForces<TYPE, kCorePoly2, 6>, 3);
-            else staged(kCompactWideForces<TYPE, 0, 6>, 3);
+            if (poly2) both(Poly2{}, Six{});
+            else both(Any{}, Six{});
         }
-        else if (poly2) staged(kCompactWideForces<TYPE, kCorePoly2, kWideCols>, 3);
-        else staged(kCompactWideForces<TYPE, 0, kWideCols>, 3);
+        else if (poly2) both(Poly2{}, All{});
+        else both(Any{}, All{});
         kCompactForces<TYPE><<<blocks, 128, 0, st>>>(m, b, kWideCap);
     }
     else
     {
-        if (poly2) staged(kCompactWideValues<TYPE, kCorePoly2>, NARROW ? 3 : 4);
-        else staged(kCompactWideValues<TYPE, 0>, NARROW ? 3 : 4);
+        bool done = false;
+        if constexpr (!NARROW)
+            if (poly2 && m.compactRows <= kGridRows && m.compactCols <= kGridCols)
+            {
+                auto grid = [&](auto cells) {
+                    constexpr int R = decltype(cells)::value;
+                    staged(kCompactGridValues<TYPE, R, kSmallCap, kSmallWarps>, small, kSmallWarps, 12, -1);
+                    staged(kCompactGridValues<TYPE, R, kWideCap, kWideWarps>, large, kWideWarps, 3, kSmallCap);
+                };
+                if (m.compactRows <= 6) grid(std::integral_constant<int, 6>{});
+                else if (m.compactRows <= 9) grid(std::integral_constant<int, 9>{});
+                else grid(std::integral_constant<int, kGridRows>{});
+                done = true;
+            }
+        if (!done)
+        {
+            auto both = [&](auto core) {
+                constexpr int C = decltype(core)::value;
+                staged(kCompactWideValues<TYPE, C, kSmallCap, kSmallWarps>, small, kSmallWarps, 16, -1);
+                staged(kCompactWideValues<TYPE, C, kWideCap, kWideWarps>, large, kWideWarps, NARROW ? 3 : 4, kSmallCap);
+            };
+            if (poly2) both(std::integral_constant<int, kCorePoly2>{});
+            else both(std::integral_constant<int, 0>{});
+        }
         kCompactValues<TYPE><<<blocks, 128, 0, st>>>(m, b, kWideCap);
     }
-    return 2;
+    return 3;
 }
 
 int launchCompactValues(DevModel const& m, BatchView const& b, int sms, cudaStream_t st)
