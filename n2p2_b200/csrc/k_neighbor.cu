@@ -8,6 +8,9 @@
 // lexicographically, with d = sqrt(dr.dr).  Every floating-point step uses
 // explicit round-to-nearest intrinsics in the reference's evaluation order
 // (Vec3D.h:294-361), so d and dr are bit-identical to the reference.
+#include <algorithm>
+#include <type_traits>
+
 #include "kernels_common.cuh"
 #include "kernels.hpp"
 
@@ -160,6 +163,7 @@ __global__ void kScatterCells(int N, const int* __restrict__ atomCell, const int
 // every lane tests a candidate whatever the cell occupancy.
 constexpr int kStencilChunk = 128;
 constexpr int kSearchWarps = 8;
+constexpr int kSplitSearch = 512, kSplitReverse = 2048;   // atoms up to which a block takes one atom
 
 struct StencilTable
 {
@@ -168,7 +172,11 @@ struct StencilTable
     int code[kStencilChunk];      // (bc0 + 512) << 20 | (bc1 + 512) << 10 | (bc2 + 512)
 };
 
-template <int PASS>
+// SPLIT: a block's eight warps share one atom, each with every eighth batch of
+// its candidates (few atoms: 192 of them leave the SMs to 24 blocks whose
+// warps walk 160 batches each, 22 us, against 8 so; the sort orders the
+// segment either way).
+template <int PASS, bool SPLIT>
 __global__ void __launch_bounds__(kSearchWarps * 32) kNeighborSearch(
     int N, double rc2, const int* __restrict__ atomStruct, const DevStructInfo* __restrict__ info,
     const double* __restrict__ px, const double* __restrict__ py, const double* __restrict__ pz,
@@ -181,10 +189,18 @@ __global__ void __launch_bounds__(kSearchWarps * 32) kNeighborSearch(
     if (PASS == 1 && guardStride > 0 && status->maxNeighbors <= guardStride) return;   // the strided search fit
     __shared__ StencilTable tables[kSearchWarps];
     StencilTable& tab = tables[threadIdx.x >> 5];
+    __shared__ int found;   // SPLIT: entries of the block's atom so far
     const int lane = threadIdx.x & 31;
-    const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += warpsPerGrid)
+    const int warpsPerGrid = SPLIT ? gridDim.x : (gridDim.x * blockDim.x) >> 5;
+    const int stride = SPLIT ? kSearchWarps * 32 : 32, begin = SPLIT ? (int)(threadIdx.x & ~31u) : 0;
+    for (int i = SPLIT ? blockIdx.x : (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += warpsPerGrid)
     {
+        if (SPLIT)
+        {
+            __syncthreads();
+            if (threadIdx.x == 0) found = 0;
+            __syncthreads();
+        }
         DevStructInfo const& s = info[atomStruct[i]];
         const double xi = px[i], yi = py[i], zi = pz[i];
         const int local = atomCell[i] - s.cellBegin;
@@ -248,7 +264,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32) kNeighborSearch(
             if (lane == 0) tab.pre[kStencilChunk] = carry;
             __syncwarp();
             const int total = carry;
-            for (int p0 = 0; p0 < total; p0 += 32)
+            for (int p0 = begin; p0 < total; p0 += stride)
             {
                 const int p = p0 + lane;
                 bool hit = false;
@@ -287,6 +303,11 @@ __global__ void __launch_bounds__(kSearchWarps * 32) kNeighborSearch(
                 {
                     const unsigned m = __ballot_sync(kFullMask, hit);
                     const int pos = __popc(m & ((1u << lane) - 1u));
+                    if (SPLIT)
+                    {
+                        if (lane == 0 && m) count = atomicAdd(&found, __popc(m));
+                        count = __shfl_sync(kFullMask, count, 0);
+                    }
                     if (hit)
                     {
                         const int64_t e = base + count + pos;
@@ -299,14 +320,20 @@ __global__ void __launch_bounds__(kSearchWarps * 32) kNeighborSearch(
                             scrDz[e] = dz;
                         }
                     }
-                    count += __popc(m);
+                    if (!SPLIT) count += __popc(m);
                 }
             }
         }
         if (PASS != 1)
         {
             if (PASS == 0) count = warpSumInt(count);   // PASS 2 counts warp-wide already
-            if (lane == 0)
+            if (SPLIT)
+            {
+                if (PASS == 0 && lane == 0) atomicAdd(&found, count);
+                __syncthreads();
+                count = found;
+            }
+            if (SPLIT ? threadIdx.x == 0 : lane == 0)
             {
                 nbrCount[i] = count;
                 atomicMax(&status->maxNeighbors, count);
@@ -433,16 +460,17 @@ __global__ void __launch_bounds__(256, 4) kNeighborSort(
 __global__ void kNeighborReverse(int N, const int* __restrict__ atomStruct, const DevStructInfo* __restrict__ info,
                                  const int64_t* __restrict__ nbrOffset, int64_t capacity,
                                  const int* __restrict__ nbrJ, const int* __restrict__ nbrCode,
-                                 int64_t* __restrict__ rev, DevStatus* __restrict__ status)
+                                 int64_t* __restrict__ rev, DevStatus* __restrict__ status, int split)
 {
-    const int lane = threadIdx.x & 31;
-    const int warpsPerGrid = (gridDim.x * blockDim.x) >> 5;
-    for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += warpsPerGrid)
+    // split: a block per atom (few atoms), else a warp
+    const int lane = split ? threadIdx.x : threadIdx.x & 31, stride = split ? blockDim.x : 32;
+    const int step = split ? gridDim.x : (gridDim.x * blockDim.x) >> 5;
+    for (int i = split ? blockIdx.x : (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < N; i += step)
     {
         if (nbrOffset[i + 1] > capacity) continue;   // overflow: the host re-runs with more room
         DevStructInfo const& s = info[atomStruct[i]];
         const int K = (2 * s.pbc[0] + 1) * (2 * s.pbc[1] + 1) * (2 * s.pbc[2] + 1);
-        for (int64_t e = nbrOffset[i] + lane; e < nbrOffset[i + 1]; e += 32)
+        for (int64_t e = nbrOffset[i] + lane; e < nbrOffset[i + 1]; e += stride)
         {
             const int j = nbrJ[e];
             if (nbrOffset[j + 1] > capacity)
@@ -620,37 +648,29 @@ void launchNeighborBuild(BatchView const& b, double rc2, cudaStream_t st)
     kScatterCells<<<blocks, 256, 0, st>>>(N, b.atomCell, b.atomSlot, b.cellStart, b.px, b.py, b.pz, b.cellAtoms,
                                           b.cellPos);
     const int warpBlocks = (N + kSearchWarps - 1) / kSearchWarps > 0 ? (N + kSearchWarps - 1) / kSearchWarps : 1;
-    if (b.scrStride > 0)
-    {
-        kNeighborSearch<2><<<warpBlocks, kSearchWarps * 32, 0, st>>>(N, rc2, b.atomStruct, b.info, b.px, b.py, b.pz,
-                                                       b.atomCell, b.cellStart, b.cellCount, b.cellPos, b.nbrCount,
-                                                       nullptr, 0, b.scrKey, b.scrD, b.scrDx, b.scrDy, b.scrDz,
-                                                       b.status, b.scrStride, 0);
-        launchExclusiveScan(N, b.nbrCount, b.nbrOffset, b.scanTmp, &b.status->totalNeighbors, st);
-        kNeighborSearch<1><<<warpBlocks, kSearchWarps * 32, 0, st>>>(N, rc2, b.atomStruct, b.info, b.px, b.py, b.pz,
-                                                       b.atomCell, b.cellStart, b.cellCount, b.cellPos, nullptr,
-                                                       b.nbrOffset,
-                                                       b.nbrCapacity, b.scrKey, b.scrD, b.scrDx, b.scrDy, b.scrDz,
-                                                       b.status, 0, b.scrStride);
-    }
-    else
-    {
-        kNeighborSearch<0><<<warpBlocks, kSearchWarps * 32, 0, st>>>(N, rc2, b.atomStruct, b.info, b.px, b.py, b.pz,
-                                                       b.atomCell, b.cellStart, b.cellCount, b.cellPos, b.nbrCount,
-                                                       nullptr, 0,
-                                                       nullptr, nullptr, nullptr, nullptr, nullptr, b.status, 0, 0);
-        launchExclusiveScan(N, b.nbrCount, b.nbrOffset, b.scanTmp, &b.status->totalNeighbors, st);
-        kNeighborSearch<1><<<warpBlocks, kSearchWarps * 32, 0, st>>>(N, rc2, b.atomStruct, b.info, b.px, b.py, b.pz,
-                                                       b.atomCell, b.cellStart, b.cellCount, b.cellPos, nullptr,
-                                                       b.nbrOffset,
-                                                       b.nbrCapacity, b.scrKey, b.scrD, b.scrDx, b.scrDy, b.scrDz,
-                                                       b.status, 0, 0);
-    }
+    // A block per atom for few atoms.  192 atoms: search 22 -> 8 us, reverse entries 11 -> 5; 1,536
+    // atoms: search 20 -> 27 (a cell's table per warp costs more than the batches saved), reverse 12 -> 11.
+    const bool split = N <= kSplitSearch, splitReverse = N <= kSplitReverse;
+    const int searchBlocks = split ? std::max(N, 1) : warpBlocks, reverseBlocks = splitReverse ? std::max(N, 1) : warpBlocks;
+    auto search = [&](auto pass, int* count, const int64_t* offset, int64_t capacity, int64_t stride, int64_t guard) {
+        constexpr int P = decltype(pass)::value;
+        auto k = split ? kNeighborSearch<P, true> : kNeighborSearch<P, false>;
+        k<<<searchBlocks, kSearchWarps * 32, 0, st>>>(N, rc2, b.atomStruct, b.info, b.px, b.py, b.pz, b.atomCell, b.cellStart,
+                                                      b.cellCount, b.cellPos, count, offset, capacity, b.scrKey, b.scrD,
+                                                      b.scrDx, b.scrDy, b.scrDz, b.status, stride, guard);
+    };
+    using Count = std::integral_constant<int, 0>;
+    using Fill = std::integral_constant<int, 1>;
+    using Strided = std::integral_constant<int, 2>;
+    if (b.scrStride > 0) search(Strided{}, b.nbrCount, nullptr, 0, b.scrStride, 0);
+    else search(Count{}, b.nbrCount, nullptr, 0, 0, 0);
+    launchExclusiveScan(N, b.nbrCount, b.nbrOffset, b.scanTmp, &b.status->totalNeighbors, st);
+    search(Fill{}, nullptr, b.nbrOffset, b.nbrCapacity, 0, b.scrStride);
     kNeighborSort<<<warpBlocks, 256, 0, st>>>(N, b.atomStruct, b.info, b.nbrOffset, b.nbrCapacity, b.scrKey, b.scrD,
                                               b.scrDx, b.scrDy, b.scrDz, b.elem, b.nbrJ, b.nbrCode, b.nbrElem,
                                               b.nbrD, b.nbrDx, b.nbrDy, b.nbrDz, b.scrStride, b.status);
-    kNeighborReverse<<<warpBlocks, 256, 0, st>>>(N, b.atomStruct, b.info, b.nbrOffset, b.nbrCapacity, b.nbrJ,
-                                                 b.nbrCode, b.rev, b.status);
+    kNeighborReverse<<<reverseBlocks, 256, 0, st>>>(N, b.atomStruct, b.info, b.nbrOffset, b.nbrCapacity, b.nbrJ,
+                                                   b.nbrCode, b.rev, b.status, splitReverse ? 1 : 0);
 }
 
 } // namespace n2p2b200
