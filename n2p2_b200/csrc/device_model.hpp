@@ -133,9 +133,12 @@ struct DevPairGroup
     int    levels;         // bit k: zeta slot k present
     int    zeta[kPairLevels];   // zeta of every slot: 1, 2, 4, 8, 16 (power-of-two form) or the group's own
     float  rc2Test;        // squared cutoff of the FP32 candidate test, rounding error added
-    float  etaScaleF[2], lambdaF[2], eta2F[2];
+    int    comp;           // numEta 1: which of the staged Gaussians is the group's
+    float  etaScaleF[2], lambdaF[2], eta2F[2], stageScaleF[2];
     double rc;
     double etaScale[2];    // -eta 64 / ln 2: argument of the table-driven exponential
+    double stageScale[2];  // the same of the two Gaussians staged per neighbour: the group's own, or those
+                           // of all the element's groups with this cutoff where they have no more than two
     double eta2[2];        // 2 eta
     double lambda[2];
     short  combo[4 * kPairLevels];   // (eta * 2 + lambda) * kPairLevels + slot -> member of the group, -1 if absent

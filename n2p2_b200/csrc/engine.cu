@@ -363,6 +363,26 @@ int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& gr
                             ++angular;
                         }
             }
+        // groups of one cutoff with two widths among them share the staged Gaussians
+        for (int k = t.begin[e]; k < t.count; ++k)
+        {
+            DevPairGroup& g = t.g[k];
+            if (g.type == 2) continue;
+            std::vector<double> scales;
+            for (int q = t.begin[e]; q < t.count; ++q)
+                if (t.g[q].type != 2 && t.g[q].cutoffSlot == g.cutoffSlot)
+                    for (int n = 0; n < t.g[q].numEta; ++n)
+                        if (std::find(scales.begin(), scales.end(), t.g[q].etaScale[n]) == scales.end())
+                            scales.push_back(t.g[q].etaScale[n]);
+            std::sort(scales.begin(), scales.end(), [](double x, double y) { return x > y; });   // ascending width
+            if (scales.size() > 2) scales.assign(g.etaScale, g.etaScale + g.numEta);
+            for (int n = 0; n < 2; ++n)
+            {
+                g.stageScale[n] = n < (int)scales.size() ? scales[n] : 0.0;
+                g.stageScaleF[n] = (float)(g.stageScale[n] / 64.0);
+            }
+            g.comp = g.numEta == 1 && scales.size() == 2 && scales[1] == g.etaScale[0] ? 1 : 0;
+        }
         t.maxAngular = std::max(t.maxAngular, angular);
     }
     for (int e = v.numElements; e <= kDevMaxElements; ++e)

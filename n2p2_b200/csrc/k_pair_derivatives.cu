@@ -106,6 +106,7 @@ __device__ __forceinline__ void angularSweep(DerivStage<CAP>& S, DevModel const&
 #pragma unroll
     for (int q = 0; q < kSweep; ++q) totG[q] = totX[q] = totY[q] = totZ[q] = 0.0;
     const double scale = G.etaScale[eta], eta2 = G.eta2[eta];
+    const int staged = G.numEta == 2 ? eta : G.comp;   // the staged Gaussian of this width
     for (int base = 0; base < owners; base += width)
     {
         const int o = base + (tid & (width - 1)), chunk = tid / width;
@@ -125,7 +126,7 @@ __device__ __forceinline__ void angularSweep(DerivStage<CAP>& S, DevModel const&
             double i1, f1, d1, e10, e11;
             S.st.geo.get(j << 4, x1, y1, z1, i1);
             S.fac.get(j << 4, f1, d1, e10, e11);
-            const double e1 = eta ? e11 : e10, i11 = i1 * i1;
+            const double e1 = staged ? e11 : e10, i11 = i1 * i1;
             for (int k = k0; k < k1; ++k)
             {
                 if (k == j) continue;
@@ -133,7 +134,7 @@ __device__ __forceinline__ void angularSweep(DerivStage<CAP>& S, DevModel const&
                 S.st.geo.get(k << 4, x2, y2, z2, i2);
                 S.fac.get(k << 4, f2, d2, e20, e21);
                 const double ri = i1 * i2, cost = (x1 * x2 + y1 * y2 + z1 * z2) * ri;
-                double V = e1 * (eta ? e21 : e20), f3 = 1.0, pr3 = 0.0;
+                double V = e1 * (staged ? e21 : e20), f3 = 1.0, pr3 = 0.0;
                 if constexpr (NARROW)
                 {
                     const double dx = x2 - x1, dy = y2 - y1, dz = z2 - z1;
@@ -288,12 +289,12 @@ __device__ __forceinline__ void atomDerivatives(DerivStage<CAP>& S, DevModel con
             radialRows<CAP>(S, model, b, gt, G, off, i);
             continue;
         }
-        if (G.cutoffSlot != slot || G.etaScale[0] != eta0 || G.etaScale[1] != eta1)
+        if (G.cutoffSlot != slot || G.stageScale[0] != eta0 || G.stageScale[1] != eta1)
         {
             __syncthreads();
             slot = G.cutoffSlot;
-            eta0 = G.etaScale[0];
-            eta1 = G.etaScale[1];
+            eta0 = G.stageScale[0];
+            eta1 = G.stageScale[1];
             const double* fc = b.nbrFc + (size_t)slot * b.nbrCapacity + off;
             const double* dfc = b.nbrDfc + (size_t)slot * b.nbrCapacity + off;
             for (int m = tid; m < n; m += kPairThreads)

@@ -17,9 +17,8 @@
 //    gets f_c = 0, so the results do not depend on the test.  Accepted pairs
 //    go to a ring per warp and are evaluated 32 at a time.
 //  * Both passes walk rounds of matchings (pair_rounds.cuh); the force pass
-//    adds a round's forces to distinct
-//    slots of the warp's own force arrays, two rounds at a time into two
-//    copies; no atomics.
+//    adds a round's forces to distinct slots of the warp's own force arrays;
+//    no atomics.
 //  * All sums run in a fixed order: results are bitwise reproducible and do
 //    not depend on the stage capacity.
 //
@@ -36,8 +35,9 @@
 // G 120 -> 26 us, forces 140 -> 33 us; 110,592 atoms with zeta up to 16 and
 // wide groups: 15.0 -> 5.4 and 17.1 -> 9.5 ms.
 // Not kept: testing rows (one j against 32
-// k) instead of rounds costs 33 % empty lanes, and run-time branches over
-// absent zeta slots cost more than summing them.
+// k) instead of rounds costs 33 % empty lanes; run-time branches over absent
+// zeta slots cost more than summing them; the accepted pairs kept in global
+// memory for the force pass save it 9 % and cost the G pass 10 %.
 #pragma once
 
 #include <type_traits>
@@ -156,10 +156,10 @@ struct GroupRegs
 };
 
 template <typename T>
-__device__ __forceinline__ T groupEtaScale(DevPairGroup const& G, int k)
+__device__ __forceinline__ T groupStageScale(DevPairGroup const& G, int k)
 {
-    if constexpr (sizeof(T) == 4) return G.etaScaleF[k];
-    else return G.etaScale[k];
+    if constexpr (sizeof(T) == 4) return G.stageScaleF[k];
+    else return G.stageScale[k];
 }
 
 template <typename T>
@@ -652,8 +652,13 @@ __device__ __forceinline__ void valuesStep(ValuesStage<T, CAP> const& S, DevPair
     S.st.geo.get(okk, x2, y2, z2, i2);
     const auto wj = pairAt<T>(S.w, oj), wk = pairAt<T>(S.w, okk);
     const T cost = (x1 * x2 + y1 * y2 + z1 * z2) * (i1 * i2);
-    T c0 = wj.x * wk.x, c1 = T(0);
-    if constexpr (TWO) c1 = wj.y * wk.y;
+    T c0, c1 = T(0);
+    if constexpr (TWO)
+    {
+        c0 = wj.x * wk.x;
+        c1 = wj.y * wk.y;
+    }
+    else c0 = G.comp ? wj.y * wk.y : wj.x * wk.x;
     if constexpr (NARROW)
     {
         const T dx = x2 - x1, dy = y2 - y1, dz = z2 - z1;
@@ -770,8 +775,8 @@ __device__ __forceinline__ void atomValues(ValuesStage<T, CAP>& S, double* parti
     auto stageFactors = [&](DevPairGroup const& G) {
         slot = G.cutoffSlot;
         factors = G.type != 2;
-        eta0 = groupEtaScale<T>(G, 0);
-        eta1 = groupEtaScale<T>(G, 1);
+        eta0 = groupStageScale<T>(G, 0);
+        eta1 = groupStageScale<T>(G, 1);
         const double* fc = b.nbrFc + (size_t)slot * b.nbrCapacity + off;
         for (int m = tid; m < n; m += kPairThreads)
         {
@@ -805,7 +810,7 @@ __device__ __forceinline__ void atomValues(ValuesStage<T, CAP>& S, double* parti
                                  warp, lane);
             continue;
         }
-        if (G.cutoffSlot != slot || !factors || groupEtaScale<T>(G, 0) != eta0 || groupEtaScale<T>(G, 1) != eta1)
+        if (G.cutoffSlot != slot || !factors || groupStageScale<T>(G, 0) != eta0 || groupStageScale<T>(G, 1) != eta1)
         {
             __syncthreads();
             stageFactors(G);
@@ -917,17 +922,19 @@ struct alignas(16) GroupCoef
     typename Pair2<T>::V w[2][kPairLevels], d[2][kPairLevels];
 };
 
-// Copies of a warp's force arrays: two rounds of matchings are added at once.
-template <int CAP>
+// Copies of a warp's force arrays: with two, two rounds of matchings are added
+// at once.  FP32 2.48 -> 2.39 ms of a force pass; in FP64 the second copy costs
+// the fifth block per SM (3.82 -> 4.02 ms).
+template <typename T, int CAP>
 constexpr int forceCopies()
 {
-    return CAP <= 384 ? 2 : 1;
+    return sizeof(T) == 4 && CAP <= 384 ? 2 : 1;
 }
 
 template <typename T, int CAP>
 struct alignas(16) ForcesStage
 {
-    static constexpr int kCopies = forceCopies<CAP>();
+    static constexpr int kCopies = forceCopies<T, CAP>();
     PairStage<T, CAP> st;
     FactorStage<T, CAP> fac;
     typename Pair2<T>::V hxy[kPairWarps][kCopies][CAP];
@@ -945,15 +952,19 @@ __device__ __forceinline__ void forcesStep(ForcesStage<T, CAP>& S, GroupCoef<T> 
     constexpr int COPIES = ForcesStage<T, CAP>::kCopies;
     using V = typename Pair2<T>::V;
     const int sj = (e >> 10) & 1023, sk = e & 1023;
-    T x1, y1, z1, i1, x2, y2, z2, i2, f1, d1, f2, d2, v0, v1;
+    T x1, y1, z1, i1, x2, y2, z2, i2, f1, d1, f2, d2, v0, v1 = T(0);
     S.st.geo.get(sj << 4, x1, y1, z1, i1);
     S.st.geo.get(sk << 4, x2, y2, z2, i2);
     {
         T a0, a1, b0, b1;
         S.fac.get(sj << 4, f1, d1, a0, a1);
         S.fac.get(sk << 4, f2, d2, b0, b1);
-        v0 = a0 * b0;
-        v1 = a1 * b1;
+        if constexpr (TWO)
+        {
+            v0 = a0 * b0;
+            v1 = a1 * b1;
+        }
+        else v0 = G.comp ? a1 * b1 : a0 * b0;
     }
     const T ri = i1 * i2;
     const T cost = (x1 * x2 + y1 * y2 + z1 * z2) * ri;
@@ -1116,8 +1127,8 @@ __device__ __forceinline__ void atomForces(ForcesStage<T, CAP>& S, GroupCoef<T>*
     T eta0 = T(0), eta1 = T(0);
     auto stageFactors = [&](DevPairGroup const& G) {
         slot = G.cutoffSlot;
-        eta0 = groupEtaScale<T>(G, 0);
-        eta1 = groupEtaScale<T>(G, 1);
+        eta0 = groupStageScale<T>(G, 0);
+        eta1 = groupStageScale<T>(G, 1);
         const double* fc = b.nbrFc + (size_t)slot * b.nbrCapacity + off;
         const double* dfc = b.nbrDfc + (size_t)slot * b.nbrCapacity + off;
         for (int m = tid; m < n; m += kPairThreads)
@@ -1133,7 +1144,7 @@ __device__ __forceinline__ void atomForces(ForcesStage<T, CAP>& S, GroupCoef<T>*
     for (int g = first; g < g1; ++g)
     {
         DevPairGroup const& G = gt.g[g];
-        if (G.cutoffSlot != slot || groupEtaScale<T>(G, 0) != eta0 || groupEtaScale<T>(G, 1) != eta1)
+        if (G.cutoffSlot != slot || groupStageScale<T>(G, 0) != eta0 || groupStageScale<T>(G, 1) != eta1)
         {
             __syncthreads();
             stageFactors(G);
