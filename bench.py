@@ -46,10 +46,10 @@ HA_TO_EV = 27.211386245988
 
 # DRAM bytes (read + write) of the two symmetry-function passes per neighbour
 # entry, from one ncu capture (dram__bytes_read.sum + dram__bytes_write.sum)
-# of the 256-box case (FP64, acceptance masks present, first tier 128 x 4),
-# all three tiers: G pass 571.3 + 118.0 MB, force pass 817.8 + 301.5 MB over
-# 13,792,482 entries; scaled to a batch by its entry count.
-SF_DRAM_BYTES_PER_ENTRY = (571.3 + 118.0 + 817.8 + 301.5) * 1e6 / 13792482
+# of the first tier of 128 boxes (FP64, stage of 160 neighbours; the other
+# tiers hold no atom): G pass 459.6 + 31.6 MB, force pass 583.3 + 243.9 MB over
+# 11.18 M entries; scaled to a batch by its entry count.
+SF_DRAM_BYTES_PER_ENTRY = (459.6 + 31.6 + 583.3 + 243.9) * 1e6 / 11.18e6
 
 # Algorithmic FLOPs per unit of the reference's symmetry-function algorithm
 # with derivatives (add/mul/div/sqrt = 1, exp counted separately):
@@ -339,12 +339,12 @@ def run_ours(args):
     roofline = None
     if fp64_peak and sf_ms > 0:
         achieved = sf_flops / (sf_ms * 1e-3) / 1e12
-        roofline = {"bound": "fp64", "kernel": "kSFValues + kSFForces (symmetry functions, values + derivatives)",
+        roofline = {"bound": "fp64", "kernel": "kPairValues + kPairForces (symmetry functions, values + derivatives)",
                     "achieved": achieved, "peak": fp64_peak, "unit": "TFLOP/s", "frac": achieved / fp64_peak,
                     "peak_source": "measured FP64 FMA throughput of this GPU (n2p2_device_fma_peak)",
                     "algorithmic_flops_per_step": sf_flops,
                     "traffic": SF_DRAM_BYTES_PER_ENTRY * work["entries"],
-                    "traffic_source": "ncu DRAM bytes of a 256-box capture, scaled by neighbour entries",
+                    "traffic_source": "ncu DRAM bytes of a 128-box capture, scaled by neighbour entries",
                     "traffic_GBps": SF_DRAM_BYTES_PER_ENTRY * work["entries"] / (sf_ms * 1e-3) / 1e9}
 
     if mixed is not None and fp32_peak:
@@ -352,7 +352,7 @@ def run_ours(args):
         ms32 = sum(t for n, t in mixed["stages_ms"].items() if n in ("sf_values", "sf_forces"))
         if ms32 > 0:
             a32 = sf_flops / (ms32 * 1e-3) / 1e12
-            mixed["roofline"] = {"bound": "fp32", "kernel": "kSFValues + kSFForces, FP32 instances",
+            mixed["roofline"] = {"bound": "fp32", "kernel": "kPairValues + kPairForces, FP32 instances",
                                  "achieved": a32, "peak": fp32_peak, "unit": "TFLOP/s", "frac": a32 / fp32_peak,
                                  "peak_source": "measured FP32 FMA throughput of this GPU (n2p2_device_fma_peak)",
                                  "algorithmic_flops_per_step": sf_flops}

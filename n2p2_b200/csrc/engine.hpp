@@ -209,9 +209,8 @@ public:
     cudaStream_t stream() const { return stream_; }
     int launchesPerEvaluate() const { return launches_; }
 
-    // Autotuning of the symmetry-function passes' first-tier shape (stage
-    // capacity x warps per block, kSFShapeCount variants): every shape of both
-    // passes is timed on this batch's own inputs and the fastest kept, or the
+    // Autotuning of the pair kernels' first-tier shape (stage capacity,
+    // kSFShapeCount variants): every shape of both passes is timed on this batch's own inputs and the fastest kept, or the
     // choice is read from the on-disk cache (N2P2_B200_TUNE_CACHE, default
     // ~/.cache/n2p2_b200/autotune.json) keyed by GPU, model plan, precision
     // and workload class.  Runs by itself before the first graph capture of a

@@ -22,22 +22,24 @@
 //  * All sums run in a fixed order: results are bitwise reproducible and do
 //    not depend on the stage capacity.
 //
-// Bound: instruction issue (G 66 %, forces 55 % of the cycles; FP64 pipe 31 %
-// and 33 %), then the latency of dependent FP64 and shared-memory
+// Bound: instruction issue (G 66 %, forces 58 % of the cycles; FP64 pipe 30 %
+// and 35 %), then the latency of dependent FP64 and shared-memory
 // instructions.  Per water atom (107 neighbours, 2548 narrow triplets, 8
 // members) the G pass executes 28.5 k warp instructions: 5.7 k staging, radial
 // functions and sums, 11 k candidates, 11.8 k triplets; the force pass 39.7 k.
 // A warp per atom (the former specialised kernels) took 56 k and 73 k: its
 // member grids had run-time exponents (selects and branches per factor) and
 // every triplet read 14 separate values.  256 water boxes (133 k atoms), FP64:
-// G 7.67 -> 4.94 ms, forces 11.1 -> 8.6 ms; mixed 5.10 -> 3.29 and 6.83 ->
-// 5.08 ms; one 192-atom box, where the four warps per atom also fill the SMs:
+// G 7.67 -> 4.9 ms, forces 11.1 -> 8.0 ms; mixed 5.10 -> 3.3 and 6.83 ->
+// 5.1 ms; one 192-atom box, where the four warps per atom also fill the SMs:
 // G 120 -> 26 us, forces 140 -> 33 us; 110,592 atoms with zeta up to 16 and
 // wide groups: 15.0 -> 5.4 and 17.1 -> 9.5 ms.
-// Not kept: testing rows (one j against 32
-// k) instead of rounds costs 33 % empty lanes; run-time branches over absent
-// zeta slots cost more than summing them; the accepted pairs kept in global
-// memory for the force pass save it 9 % and cost the G pass 10 %.
+// Not kept: testing rows (one j against 32 k) instead of rounds costs 33 %
+// empty lanes; run-time branches over absent zeta slots cost more than summing
+// them; the accepted pairs kept in global memory for the force pass save it
+// 9 % and cost the G pass 10 %; warp shares that are not multiples of 64
+// candidates, and the groups' short blocks started at different warps, change
+// nothing (G 2.33 and 2.32 ms, forces 3.82 and 3.82 ms for 96 boxes).
 #pragma once
 
 #include <type_traits>

@@ -261,12 +261,13 @@ def gaussian_bases(etas):
 
 def specialised_kernel_admissible(sfs):
     """admissible(chosen, j) for greedy_span_selection: adding candidate j
-    keeps every group of the chosen set runnable by the model-specialised
-    symmetry-function kernels -- radial groups (per neighbour element and
+    keeps every group of the chosen set cheap on the pair kernels of the
+    symmetry functions -- radial groups (per neighbour element and
     cutoff) with at most GAUSSIAN_PLAN_MAX_BASES base Gaussians; angular
     groups (per element pair and cutoff) with one base Gaussian, at most two
-    widths, two lambdas and four integer zetas <= 32.  A descriptor outside
-    this runs on the generic kernels, several times slower per triplet.
+    widths, two lambdas and four integer zetas <= 32.  (Shifted angular
+    functions and zeta above 31 run the general kernels, several times slower
+    per triplet.)
     sfs: Mode.symmetryFunction tuples of the candidates."""
     def key(f):
         return (f[0], f[1], f[2] if f[0] != 2 else -1, f[7])
