@@ -187,6 +187,10 @@ namespace {
 // neuron, reading a weight once (through the read-only cache: every block of
 // an element reads the same matrices) for UNIT fused multiply-adds.  Every sum
 // runs over the reduction index in ascending order, as in propagateLayer.
+// Bound by latency and the weights' loads, so by the blocks that fit an SM: only the
+// first activation buffer has the inputs' width, the other three the hidden layers'
+// (40-25-25-1 networks of 133 k atoms 527 -> 380 us; 354-30-20-1 networks, which a
+// tile did not hold before, 151 us by kNetworkFP64 -> 96 us for 4,096 atoms).
 constexpr int kNetThreads = 128;
 
 // Row of a tile of TILE atoms: padded by four against bank conflicts (rows stay 32-byte aligned).
@@ -195,10 +199,11 @@ __host__ __device__ constexpr int netRow() { return TILE + 4; }
 
 __host__ __device__ inline int netSmemDoubles(DevElement const& E, int row)
 {
-    int maxW = 0, sumD = 0;
-    for (int l = 0; l < E.numLayers; ++l) maxW = E.neurons[l] > maxW ? E.neurons[l] : maxW;
+    int maxH = 0, sumD = 0;
+    for (int l = 1; l < E.numLayers; ++l) maxH = E.neurons[l] > maxH ? E.neurons[l] : maxH;
     for (int l = 1; l < E.numLayers; ++l) sumD += E.neurons[l];
-    return (2 * maxW + sumD + 2 * maxW) * row;   // activations, derivatives per layer, reverse vectors
+    const int maxW = E.neurons[0] > maxH ? E.neurons[0] : maxH;
+    return (maxW + maxH + sumD + 2 * maxH) * row;   // activations (inputs; layers), derivatives per layer, reverse vectors
 }
 
 // Sum over the reduction index r < n of w(r) x[r][a] for the unit's UNIT
@@ -286,16 +291,17 @@ __global__ void __launch_bounds__(kNetThreads, 3) kNetworkTiled(DevModel model, 
         const int L = E.numLayers;
         const int first = b.elemBegin[e] + (tile - tilesOf[e]) * TILE;
         const int count = min(TILE, b.elemBegin[e + 1] - first);
-        int maxW = 0;
-        for (int l = 0; l < L; ++l) maxW = max(maxW, E.neurons[l]);
+        int maxH = 0;
+        for (int l = 1; l < L; ++l) maxH = max(maxH, E.neurons[l]);
+        const int maxW = max(maxH, E.neurons[0]);
         double* act[2] = {sm, sm + maxW * netRow<TILE>()};
-        double* dfBase = sm + 2 * maxW * netRow<TILE>();
+        double* dfBase = sm + (maxW + maxH) * netRow<TILE>();
         double* gv[2];
         {
             int sumD = 0;
             for (int l = 1; l < L; ++l) sumD += E.neurons[l];
             gv[0] = dfBase + sumD * netRow<TILE>();
-            gv[1] = gv[0] + maxW * netRow<TILE>();
+            gv[1] = gv[0] + maxH * netRow<TILE>();
         }
         __syncthreads();   // the previous tile's reads of the buffers are done (its output may sit in act[0])
         // the tile's G rows, neuron-major (atoms beyond the element's last: zeros)
