@@ -1412,8 +1412,14 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
     if (stages & STAGE_NETWORKS)
     {
         // The tensor-core networks take 46 us however few their 128-atom tiles are; below a tile of 32 per
-        // SM the FP64 kernel is faster (1,536 atoms: 18 us) and exact.
-        const bool few = (N_ + 31) / 32 < sms_;
+        // SM the FP64 kernel is faster for small networks (1,701 weights, 1,536 atoms: 18 us) and exact.
+        // Networks of 7,873 weights are not: with them a mixed call took 548 us instead of 507.
+        bool few = (N_ + 31) / 32 < sms_;
+        for (int e = 0; e < m.numElements; ++e)
+        {
+            DevElement const& E = m.el[e];
+            few = few && E.bOffset[E.numLayers - 1] + E.neurons[E.numLayers - 1] - E.wOffset[1] <= 2048;
+        }
         if (precision == PREC_MIXED && dmodel_.tcNetwork && !few) launchNetworkTC(m, v_, forces ? 1 : 0, sms_, stream_);
         else launchNetworkFP64(m, v_, forces ? 1 : 0, sms_, stream_);
         launches += 1;
