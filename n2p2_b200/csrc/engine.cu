@@ -1413,7 +1413,7 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
     {
         // The tensor-core networks take 46 us however few their 128-atom tiles are; below a tile of 32 per
         // SM the FP64 kernel is faster for small networks (1,701 weights, 1,536 atoms: 18 us) and exact.
-        // Networks of 7,873 weights are not: with them a mixed call took 548 us instead of 507.
+        // Larger ones keep the tensor cores: the FP64 time grows with the weights, theirs hardly.
         bool few = (N_ + 31) / 32 < sms_;
         for (int e = 0; e < m.numElements; ++e)
         {
