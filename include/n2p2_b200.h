@@ -244,7 +244,8 @@ n2p2_status n2p2_batch_get_neighbors(n2p2_batch* batch, int64_t* offsets, int32_
                                      double* d, double* dr);
 
 /* Atom::G, Atom::dEdG (concatenated per atom, numSymmetryFunctions values each)
- * and Atom::energy (internal units). */
+ * and Atom::energy (internal units).  Several threads may read G and dE/dG of
+ * one evaluated batch at once. */
 n2p2_status n2p2_batch_get_symmetry_functions(n2p2_batch* batch, double* G);
 n2p2_status n2p2_batch_get_dEdG(n2p2_batch* batch, double* dEdG);
 n2p2_status n2p2_batch_get_atomic_energies(n2p2_batch* batch, double* energies);

@@ -1960,7 +1960,7 @@ void Batch::copyNeighbors(int64_t* offsets, int* index, int* image, double* d, d
 // (every atom's functions in turn).  The caller's memory is pageable and often
 // untouched, so one thread spends most of the time in page faults: up to
 // kPackThreads threads take ranges of atoms, each through a slice of the
-// batch's page-locked staging in pieces.  67 k atoms x 40 functions (21 MB):
+// batch's page-locked staging in pieces (the caller holds readMutex_).  67 k atoms x 40 functions (21 MB):
 // 11 ms as one copy to a host vector packed by one thread, 1.5 ms so.  A few
 // pieces or less go through a vector.
 constexpr int kPackThreads = 8;
@@ -2036,6 +2036,7 @@ void Batch::copyPerAtom(const double* dev, double* out)
 
 void Batch::copyG(double* out)
 {
+    std::lock_guard<std::mutex> lock(readMutex_);
     verify();
     synchronize();
     copyPerAtom(v_.G, out);
@@ -2043,6 +2044,7 @@ void Batch::copyG(double* out)
 
 void Batch::copyDEdG(double* out)
 {
+    std::lock_guard<std::mutex> lock(readMutex_);
     verify();
     synchronize();
     copyPerAtom(v_.dEdG, out);

@@ -4,6 +4,7 @@
 
 #include <cstdint>
 #include <map>
+#include <mutex>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -272,6 +273,7 @@ private:
                 int stages = STAGE_ALL);
     void symmetryFunctionPass(int pass, int precision, int variant);
     void copyPerAtom(const double* dev, double* out);
+    std::mutex readMutex_;          // one reader of per-atom results at a time: they share packStage_
     double* packStage_ = nullptr;   // page-locked staging of copyPerAtom, allocated at its first large copy
     DevStatus readStatus();   // the device status word as it is (synchronises)
     void releaseGraph();
