@@ -45,7 +45,9 @@ typedef int n2p2_status;
 
 /* Precision of the symmetry-function and network stages. */
 #define N2P2_PRECISION_FP64 0       /* plain FP64 throughout                          */
-#define N2P2_PRECISION_MIXED 1      /* FP32 descriptors, FP64 cutoff/scaling/sums     */
+#define N2P2_PRECISION_MIXED 1      /* FP32 descriptors, FP64 cutoff/scaling/sums;
+                                       networks by the model alone: FP64 up to 2,048
+                                       parameters per element, else tensor cores      */
 
 /* Flags of n2p2_batch_evaluate. */
 #define N2P2_EVAL_FORCES 1          /* Mode::evaluateNNP(useForces = true)            */

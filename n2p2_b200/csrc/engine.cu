@@ -837,7 +837,22 @@ void DeviceModel::upload(Model const& m)
     mix(&v.sortByDistance, sizeof(int));
     mix(v.cutoff, sizeof(v.cutoff));
     fingerprint = h;
-    tcNetwork = networkTCSupported(m);
+    // Networks of the mixed form: a choice of the model alone, so that a structure's energy depends
+    // neither on its batch nor on a rank's number of atoms (the tensor-core form is off by up to
+    // 0.1 meV per atom, part of it systematic).  Up to kExactParameters per element the FP64 kernels:
+    // 1,701 parameters take them 23 to 26 us for 192 to 4,320 atoms (tensor cores 50: a chain of
+    // four products and their waits, however few the tiles) and 520 us for 138 k (344), of whole
+    // calls of 200 us and 11.2 ms; 945 parameters 20 us (35) and 430 us (217).  Above it the tensor cores:
+    // 4,369 parameters 37 us (70) for 192 atoms, but 995 (492) of 11.4 ms for 138 k; 6,849 43 (88)
+    // and 1,165 (621).
+    constexpr int kExactParameters = 2048;
+    bool small = true;
+    for (int e = 0; e < v.numElements; ++e)
+    {
+        DevElement const& E = v.el[e];
+        small = small && E.bOffset[E.numLayers - 1] + E.neurons[E.numLayers - 1] - E.wOffset[1] <= kExactParameters;
+    }
+    tcNetwork = networkTCSupported(m) && !small;
     v.weightsT = weightsT_;
     view = v;
     this->maxSF = maxSF;
@@ -1411,16 +1426,7 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
     }
     if (stages & STAGE_NETWORKS)
     {
-        // The tensor-core networks take 46 us however few their 128-atom tiles are; below a tile of 32 per
-        // SM the FP64 kernel is faster for small networks (1,701 weights, 1,536 atoms: 18 us) and exact.
-        // Larger ones keep the tensor cores: the FP64 time grows with the weights, theirs hardly.
-        bool few = (N_ + 31) / 32 < sms_;
-        for (int e = 0; e < m.numElements; ++e)
-        {
-            DevElement const& E = m.el[e];
-            few = few && E.bOffset[E.numLayers - 1] + E.neurons[E.numLayers - 1] - E.wOffset[1] <= 2048;
-        }
-        if (precision == PREC_MIXED && dmodel_.tcNetwork && !few) launchNetworkTC(m, v_, forces ? 1 : 0, sms_, stream_);
+        if (precision == PREC_MIXED && dmodel_.tcNetwork) launchNetworkTC(m, v_, forces ? 1 : 0, sms_, stream_);
         else launchNetworkFP64(m, v_, forces ? 1 : 0, sms_, stream_);
         launches += 1;
         mark("network");

@@ -62,7 +62,7 @@ public:
     int maxSF = 0;
     size_t numWeights = 0;               // entries of the flat weight array
     uint64_t fingerprint = 0;            // hash of the evaluation plan (groups, members, cutoffs)
-    bool tcNetwork = false;              // mixed form runs the networks on the tensor cores
+    bool tcNetwork = false;              // the mixed form runs the model's networks on the tensor cores
     bool networksSet = true;             // every element has weights (else symmetry functions only)
     std::string missingWeights;
     double* weightsDevice() const { return weights_; }
