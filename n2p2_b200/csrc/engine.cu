@@ -250,7 +250,7 @@ namespace {
 // kPairLevels zeta slots (the pairs are enumerated again for every part).
 // Returns DevModel::pairForm, 0 when the kernels of sf_fast.cuh must run the
 // model: an angular function with a shift or a zeta that is no integer (or
-// beyond powAny's 31), a function listed twice, a Gaussian that leaves the
+// beyond 32, the largest tested), a function listed twice, a Gaussian that leaves the
 // range of the table-driven exponential (2^-1000), or more groups than the
 // kernels' argument holds.
 int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& groups,
@@ -265,7 +265,7 @@ int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& gr
             const double reach = g.rc + std::fabs(M.rs);
             if (!(M.eta >= 0.0) || M.eta * reach * reach * log2e > 1000.0) return 0;
             if (g.type == 2) continue;
-            if (M.rs != 0.0 || !M.useIntPow || M.zetaInt < 1 || M.zetaInt > 31) return 0;
+            if (M.rs != 0.0 || !M.useIntPow || M.zetaInt < 1 || M.zetaInt > 32) return 0;
             const int z = M.zetaInt;
             pow16 = pow16 && (z == 1 || z == 2 || z == 4 || z == 8 || z == 16);
             // |lambda| > 1: 1 + lambda cos may be negative, and such terms vanish (general form)

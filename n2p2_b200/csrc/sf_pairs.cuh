@@ -171,7 +171,7 @@ __device__ __forceinline__ T groupEta2(DevPairGroup const& G, int k)
     else return G.eta2[k];
 }
 
-// x^n, 0 <= n <= 31 warp-uniform.
+// x^n, n >= 0 warp-uniform.
 template <typename T>
 __device__ __forceinline__ T powAny(T x, int n)
 {

@@ -266,7 +266,7 @@ def specialised_kernel_admissible(sfs):
     cutoff) with at most GAUSSIAN_PLAN_MAX_BASES base Gaussians; angular
     groups (per element pair and cutoff) with one base Gaussian, at most two
     widths, two lambdas and four integer zetas <= 32.  (Shifted angular
-    functions and zeta above 31 run the general kernels, several times slower
+    functions and zeta above 32 run the general kernels, several times slower
     per triplet.)
     sfs: Mode.symmetryFunction tuples of the candidates."""
     def key(f):
