@@ -208,7 +208,7 @@ struct DevModel
     int normalizeNeurons;
     int sortByDistance;   // an angular group has a cutoff below the largest: stage blocks sorted by r
     int pairForm;         // the pair kernels run the model (DevPairTable): 0 no, 1 every zeta a power of two <= 4,
-                          // 2 <= 16, 3 other integers
+                          // 2 <= 16, 3 other integers, 4 any integers, angular Gaussians that underflow inside the cutoff
     const double* expTable;   // 2^(j/64), j < 64
     double maxCutoff, maxCutoff2;
     DevElement el[kDevMaxElements];

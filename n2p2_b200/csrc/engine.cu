@@ -250,21 +250,26 @@ namespace {
 // kPairLevels zeta slots (the pairs are enumerated again for every part).
 // Returns DevModel::pairForm, 0 when the kernels of sf_fast.cuh must run the
 // model: an angular function with a shift or a zeta that is no integer (or
-// beyond 32, the largest tested), a function listed twice, a Gaussian that leaves the
-// range of the table-driven exponential (2^-1000), or more groups than the
-// kernels' argument holds.
+// beyond 32, the largest tested), a function listed twice, an exponent beyond
+// 2^24 inside the cutoff, or more groups than the kernels' argument holds.
+// One radial function of eta 6 beside the 40 of the water model (33 k atoms):
+// G 5.76 and forces 5.66 ms there, 1.31 and 2.07 here; one angular width of
+// eta 6: 13.2 and 9.8, here 4.8 and 6.9.
 int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& groups,
               std::vector<DevMember> const& members, DevPairTable& t)
 {
     const double log2e = 1.0 / std::log(2.0);
-    bool pow4 = true, pow16 = true;
+    bool pow4 = true, pow16 = true, wide = false;
     for (DevGroup const& g : groups)
         for (int q = g.memberBegin; q < g.memberBegin + g.memberCount; ++q)
         {
             DevMember const& M = members[q];
-            const double reach = g.rc + std::fabs(M.rs);
-            if (!(M.eta >= 0.0) || M.eta * reach * reach * log2e > 1000.0) return 0;
+            // largest |r - rs|, 0 <= r <= rc; expScaled takes exponents up to 2^30 / 64
+            const double reach = std::max(std::fabs(M.rs), std::fabs(g.rc - M.rs));
+            const double exponent = M.eta * reach * reach * log2e;
+            if (!(M.eta >= 0.0) || exponent > 16777216.0) return 0;
             if (g.type == 2) continue;
+            wide = wide || exponent > 1000.0;
             if (M.rs != 0.0 || !M.useIntPow || M.zetaInt < 1 || M.zetaInt > 32) return 0;
             const int z = M.zetaInt;
             pow16 = pow16 && (z == 1 || z == 2 || z == 4 || z == 8 || z == 16);
@@ -272,7 +277,7 @@ int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& gr
             pow16 = pow16 && std::fabs(M.lambda) <= 1.0;
             pow4 = pow4 && z <= 4;
         }
-    const int form = !pow16 ? 3 : pow4 ? 1 : 2;
+    const int form = wide ? 4 : !pow16 ? 3 : pow4 ? 1 : 2;
     int member = 0, radials = 0;
     for (int e = 0; e < v.numElements; ++e)
     {
@@ -323,7 +328,7 @@ int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& gr
                 }
                 std::sort(etas.begin(), etas.end());
                 std::sort(zetas.begin(), zetas.end());
-                if (form != 3) zetas = {1, 2, 4, 8, 16};
+                if (form <= 2) zetas = {1, 2, 4, 8, 16};
                 for (size_t a = 0; a < etas.size(); a += 2)
                     for (size_t l = 0; l < lams.size(); l += 2)
                         for (size_t z = 0; z < zetas.size(); z += kPairLevels)

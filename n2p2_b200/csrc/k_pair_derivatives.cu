@@ -143,7 +143,7 @@ __device__ __forceinline__ void angularSweep(DerivStage<CAP>& S, DevModel const&
                     double d3;
                     pairCutoff<CUT>(cut, cut.iw, s * i3, f3, d3);
                     if (f3 == 0.0 && d3 == 0.0) continue;
-                    V *= expScaled(s, scale, S.st.expTab);
+                    V *= expScaled<CUT == kCutAny>(s, scale, S.st.expTab);
                     pr3 = f1 * f2 * d3 * i3;
                 }
                 const double pfc = f1 * f2 * f3, A3 = pfc * ri, A1 = pfc * (ri - cost * i11);
@@ -243,7 +243,7 @@ __device__ __forceinline__ void radialRows(DerivStage<CAP>& S, DevModel const& m
                 DevRadial const& R = rad[m0 + q];
                 DevMember const& M = mem[m0 + q];
                 const double d = r - R.rs;
-                const double v = expScaled(d * d, R.scale, S.st.expTab);
+                const double v = expScaled<true>(d * d, R.scale, S.st.expTab);
                 const double p1 = (df - R.eta2 * d * f) * v * ri;
                 totG[q] += v * f;
                 totX[q] += p1 * x;
@@ -301,7 +301,7 @@ __device__ __forceinline__ void atomDerivatives(DerivStage<CAP>& S, DevModel con
             {
                 const int s = S.st.slotOf[m];
                 const double r = S.st.geo.r[s], r2 = r * r;
-                S.fac.set(s, fc[m], dfc[m] / r, expScaled(r2, eta0, S.st.expTab), expScaled(r2, eta1, S.st.expTab));
+                S.fac.set(s, fc[m], dfc[m] / r, expScaled<CUT == kCutAny>(r2, eta0, S.st.expTab), expScaled<CUT == kCutAny>(r2, eta1, S.st.expTab));
             }
             __syncthreads();
         }
@@ -360,7 +360,7 @@ void derivativesTier(DevModel const& m, DevPairTable const& gt, BatchView const&
 void launchPairDerivatives(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st)
 {
     const int need = (b.N + kPairThreads - 1) / kPairThreads, tier = need < sms ? need : sms;
-    if (m.cutoff[0].type == kCutPoly2 && m.cutoff[0].rci == 0.0)
+    if (m.pairForm <= 3 && m.cutoff[0].type == kCutPoly2 && m.cutoff[0].rci == 0.0)
     {
         derivativesTier<kDerivCap, kCutPoly2, false>(m, gt, b, b.N, -1, st);
         derivativesTier<kDerivBigCap, kCutPoly2, true>(m, gt, b, tier, kDerivCap, st);

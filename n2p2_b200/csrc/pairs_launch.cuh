@@ -60,7 +60,8 @@ void pairForces(DevModel const& m, DevPairTable const& gt, BatchView const& b, i
 }
 
 // Instances: the poly2 cutoff with zeta powers of two up to 4 or 16, any
-// cutoff with powers of two, and any integers.
+// cutoff with powers of two, and any integers (the only one for angular
+// Gaussians that underflow inside the cutoff, pairForm 4).
 template <typename T>
 void pairValuesT(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant)
 {

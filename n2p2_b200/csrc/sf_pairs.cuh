@@ -70,15 +70,21 @@ constexpr double kLn64 = 0.69314718055994530942 / 64.0;
 __constant__ double kExpCoef[5] = {kLn64, kLn64* kLn64 / 2.0, kLn64* kLn64* kLn64 / 6.0,
                                    kLn64* kLn64* kLn64* kLn64 / 24.0, kLn64* kLn64* kLn64* kLn64* kLn64 / 120.0};
 
-// exp(-eta s) as 2^(c s / 64), c = -eta 64 / ln 2, -1000 <= c s / 64 <= 0:
+// exp(-eta s) as 2^(c s / 64), c = -eta 64 / ln 2, -2^30 <= c s <= 0:
 // table-driven exponential (P. T. P. Tang, ACM TOMS 15 (1989) 144): c s =
 // k + f with |f| <= 1/2, 2^(k/64) from the 64-entry table and k's upper bits,
-// 2^(f/64) - 1 by its series to order 5 (truncation 3.5e-17).
+// 2^(f/64) - 1 by its series to order 5 (truncation 3.5e-17).  WIDE false:
+// c s / 64 >= -1000; true: below 2^-1021 the result is 2^-1021 instead of the
+// underflowing value (one instruction more: in every triplet it costs the
+// passes 1 to 4 %, so only the radial functions and the instances for any
+// zeta have it).
+template <bool WIDE = false>
 __device__ __forceinline__ double expScaled(double s, double c, const double* tab)
 {
     constexpr double kShift = 6755399441055744.0;   // 1.5 2^52: adding it rounds to an integer
     double kd = fma(s, c, kShift);
-    const int k = __double2loint(kd);
+    int k = __double2loint(kd);
+    if (WIDE) k = max(k, -64 * 1021);
     kd -= kShift;
     const double f = fma(s, c, -kd);
     const double p = f * fma(f, fma(f, fma(f, fma(f, kExpCoef[4], kExpCoef[3]), kExpCoef[2]), kExpCoef[1]), kExpCoef[0]);
@@ -88,6 +94,7 @@ __device__ __forceinline__ double expScaled(double s, double c, const double* ta
 }
 
 // FP32 form: c = -eta / ln 2.
+template <bool WIDE = false>
 __device__ __forceinline__ float expScaled(float s, float c, const double*)
 {
     float r;
@@ -669,8 +676,8 @@ __device__ __forceinline__ void valuesStep(ValuesStage<T, CAP> const& S, DevPair
         T f, df;
         pairCutoff<CUT>(cut, R.iw, r, f, df);
         if (!ok) f = T(0);
-        c0 *= f * expScaled(s, R.scale0, S.st.expTab);
-        if constexpr (TWO) c1 *= f * expScaled(s, R.scale1, S.st.expTab);
+        c0 *= f * expScaled<FORM == 0>(s, R.scale0, S.st.expTab);
+        if constexpr (TWO) c1 *= f * expScaled<FORM == 0>(s, R.scale1, S.st.expTab);
     }
     else if (!ok) c0 = c1 = T(0);
 #pragma unroll
@@ -749,7 +756,7 @@ __device__ __forceinline__ void valuesRadial(ValuesStage<T, CAP>& S, double* par
                 {
                     DevRadial const& M = rad[m0 + q];
                     const T d = r - radialShift<T>(M);
-                    v[q] += expScaled(d * d, radialScale<T>(M), S.st.expTab) * fc;
+                    v[q] += expScaled<true>(d * d, radialScale<T>(M), S.st.expTab) * fc;
                 }
             }
         }
@@ -789,8 +796,8 @@ __device__ __forceinline__ void atomValues(ValuesStage<T, CAP>& S, double* parti
             {
                 const T r = S.st.geo.r[s], r2 = r * r;
                 typename Pair2<T>::V w;
-                w.x = f * expScaled(r2, eta0, S.st.expTab);
-                w.y = f * expScaled(r2, eta1, S.st.expTab);
+                w.x = f * expScaled<FORM == 0>(r2, eta0, S.st.expTab);
+                w.y = f * expScaled<FORM == 0>(r2, eta1, S.st.expTab);
                 S.w[s] = w;
             }
         }
@@ -978,8 +985,8 @@ __device__ __forceinline__ void forcesStep(ForcesStage<T, CAP>& S, GroupCoef<T> 
         const T i3 = invSqrt(s);
         pairCutoff<CUT>(cut, R.iw, s * i3, f3, d3);
         d3 *= i3;
-        v0 *= expScaled(s, R.scale0, S.st.expTab);
-        if constexpr (TWO) v1 *= expScaled(s, R.scale1, S.st.expTab);
+        v0 *= expScaled<FORM == 0>(s, R.scale0, S.st.expTab);
+        if constexpr (TWO) v1 *= expScaled<FORM == 0>(s, R.scale1, S.st.expTab);
     }
     T Q0 = T(0), R0 = T(0), Q1 = T(0), R1 = T(0);
 #pragma unroll
@@ -1137,8 +1144,8 @@ __device__ __forceinline__ void atomForces(ForcesStage<T, CAP>& S, GroupCoef<T>*
         {
             const int s = S.st.slotOf[m];
             const T r = S.st.geo.r[s], r2 = r * r;
-            S.fac.set(s, (T)fc[m], (T)(dfc[m] / b.nbrD[off + m]), expScaled(r2, eta0, S.st.expTab),
-                      expScaled(r2, eta1, S.st.expTab));
+            S.fac.set(s, (T)fc[m], (T)(dfc[m] / b.nbrD[off + m]), expScaled<FORM == 0>(r2, eta0, S.st.expTab),
+                      expScaled<FORM == 0>(r2, eta1, S.st.expTab));
         }
     };
     if (first < g1) stageFactors(gt.g[first]);
@@ -1201,7 +1208,7 @@ __device__ __forceinline__ void atomForces(ForcesStage<T, CAP>& S, GroupCoef<T>*
             for (int q = 0; q < G.memberCount; ++q)
             {
                 const T d = r - radialShift<T>(rad[q]);
-                const T v = expScaled(d * d, radialScale<T>(rad[q]), S.st.expTab);
+                const T v = expScaled<true>(d * d, radialScale<T>(rad[q]), S.st.expTab);
                 P += (T)c[q] * (dfc - radialEta2<T>(rad[q]) * d * fc) * v;
             }
         }

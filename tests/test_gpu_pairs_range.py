@@ -1,6 +1,8 @@
 """The ends of the pair kernels' range of functions (sf_pairs.cuh): zeta up to
-32.  They run there (no candidate_masks stage, which only the general kernels
-have), with the C restatement's energies and forces.
+32, Gaussians that underflow inside the cutoff (eta r^2 log2 e beyond the
+exponent range of a double, shifted and not, radial, narrow and wide) and
+shifts far out.  They run there (no candidate_masks stage, which only the
+general kernels have), with the C restatement's energies and forces.
 
 Tolerances: those of the other parity tests, 1e-10 of the energy and of the
 largest force component."""
@@ -16,9 +18,15 @@ pytestmark = pytest.mark.gpu
 PAIRS = (("H", "H"), ("H", "O"), ("O", "O"))
 RADIAL = [(0.01, 0.0), (0.3, 1.5)]
 PLAIN = [(3, 0.01, 1, 4)]
+# cutoff 12: eta r_c^2 log2 e is 208 eta
 FORMS = {
     "zeta31": (RADIAL, PLAIN + [(3, 0.01, 1, 31), (9, 0.01, -1, 31)]),
     "zeta32": (RADIAL, PLAIN + [(3, 0.01, 1, 32), (3, 0.01, -1, 32), (9, 0.02, 1, 32), (9, 0.02, 1, 16)]),
+    "at_1000": (RADIAL + [(4.8, 0.0), (4.82, 0.0)], PLAIN),
+    "wide_radial": (RADIAL + [(6.0, 0.0), (20.0, 0.0), (30.0, 2.0)], PLAIN),
+    "far_shift": (RADIAL + [(2.0, 9.0), (4.0, 6.0), (3.0, 11.5)], PLAIN),
+    "wide_narrow": (RADIAL, PLAIN + [(3, 5.0, 1, 2), (3, 8.0, -1, 1)]),
+    "wide_wide": (RADIAL, PLAIN + [(9, 7.0, 1, 1), (9, 7.0, -1, 3)]),
 }
 
 
