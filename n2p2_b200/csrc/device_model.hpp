@@ -131,7 +131,9 @@ struct DevPairGroup
     int    radialBegin;    // radial groups: their members in DevPairTable::radial
     int    numEta;
     int    levels;         // bit k: zeta slot k present
-    int    zeta[kPairLevels];   // zeta of every slot: 1, 2, 4, 8, 16 (power-of-two form) or the group's own
+    int    zeta[kPairLevels];   // zeta of every slot: 1, 2, 4, 8, 16 (power-of-two form), 1, 2, 3, 4 (cubic) or
+                                // the group's own
+    int    cubic;
     float  rc2Test;        // squared cutoff of the FP32 candidate test, rounding error added
     int    comp;           // numEta 1: which of the staged Gaussians is the group's
     float  etaScaleF[2], lambdaF[2], eta2F[2], stageScaleF[2];

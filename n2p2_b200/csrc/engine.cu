@@ -260,7 +260,10 @@ int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& gr
 {
     const double log2e = 1.0 / std::log(2.0);
     bool pow4 = true, pow16 = true, wide = false;
-    for (DevGroup const& g : groups)
+    std::vector<char> cubic(groups.size(), 1);   // zeta 1 to 4, and no term with 1 + lambda cos < 0
+    for (size_t k = 0; k < groups.size(); ++k)
+    {
+        DevGroup const& g = groups[k];
         for (int q = g.memberBegin; q < g.memberBegin + g.memberCount; ++q)
         {
             DevMember const& M = members[q];
@@ -276,7 +279,9 @@ int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& gr
             // |lambda| > 1: 1 + lambda cos may be negative, and such terms vanish (general form)
             pow16 = pow16 && std::fabs(M.lambda) <= 1.0;
             pow4 = pow4 && z <= 4;
+            if (z > 4 || std::fabs(M.lambda) > 1.0) cubic[k] = 0;
         }
+    }
     const int form = wide ? 4 : !pow16 ? 3 : pow4 ? 1 : 2;
     int member = 0, radials = 0;
     for (int e = 0; e < v.numElements; ++e)
@@ -328,7 +333,9 @@ int planPairs(Model const& m, DevModel const& v, std::vector<DevGroup> const& gr
                 }
                 std::sort(etas.begin(), etas.end());
                 std::sort(zetas.begin(), zetas.end());
+                p.cubic = form == 3 && cubic[k];
                 if (form <= 2) zetas = {1, 2, 4, 8, 16};
+                if (p.cubic) zetas = {1, 2, 3, 4};
                 for (size_t a = 0; a < etas.size(); a += 2)
                     for (size_t l = 0; l < lams.size(); l += 2)
                         for (size_t z = 0; z < zetas.size(); z += kPairLevels)

@@ -609,13 +609,21 @@ __device__ __forceinline__ void forTierAtoms(unsigned* todo, BatchView const& b,
 }
 
 // f(narrow, form) for a group of a model of form FORM: models with zeta up
-// to 16 run the groups with zeta up to 4 in the shorter form.
+// to 16 run the groups with zeta up to 4 in the shorter form, models with any
+// integers those with zeta 1 to 4 in a form of their own (zeta {1, 3}, 33 k
+// atoms: in the any-integer form G takes 2.48 and the forces 2.95 ms, in this
+// one 1.61 and 2.53).
 template <int FORM, typename F>
 __device__ __forceinline__ void withForm(DevPairGroup const& G, F f)
 {
     using True = std::integral_constant<bool, true>;
     using False = std::integral_constant<bool, false>;
-    if (FORM == 5 && !(G.levels >> 3))
+    if (FORM == 0 && G.cubic)
+    {
+        if (G.type == 3) f(True{}, std::integral_constant<int, 4>{});
+        else f(False{}, std::integral_constant<int, 4>{});
+    }
+    else if (FORM == 5 && !(G.levels >> 3))
     {
         if (G.type == 3) f(True{}, std::integral_constant<int, 3>{});
         else f(False{}, std::integral_constant<int, 3>{});
@@ -649,7 +657,7 @@ __device__ __forceinline__ typename Pair2<T>::V pairAt(typename Pair2<T>::V cons
 // One step of a warp: 32 accepted pairs (lanes past `take` repeat the first
 // one with weight 0).  acc[(eta * 2 + lambda) * Z + slot] += G terms.
 // FORM 3, 5: zeta 2^slot (slots up to 4, 16), absent ones summed as well;
-// 0: any zeta, five slots.  TWO: the group has two etas.
+// 4: zeta 1 to 4; 0: any zeta, five slots.  TWO: the group has two etas.
 template <typename T, int CAP, int CUT, bool NARROW, int FORM, bool TWO>
 __device__ __forceinline__ void valuesStep(ValuesStage<T, CAP> const& S, DevPairGroup const& G, GroupRegs<T> const& R,
                                            DevCutoff const& cut, int e, bool ok, T* acc)
@@ -685,12 +693,13 @@ __device__ __forceinline__ void valuesStep(ValuesStage<T, CAP> const& S, DevPair
     {
         T p = T(1) + (l ? R.lam1 : R.lam0) * cost;
         if constexpr (FORM == 0) p = clampZero(p);
+        const T p1 = p;
 #pragma unroll
         for (int z = 0; z < Z; ++z)
         {
-            if (FORM && z > 0) p = p * p;
+            if (FORM && z > 0 && !(FORM == 4 && z == 2)) p = p * p;
             if (FORM == 0 && !(G.levels >> z & 1)) continue;
-            const T q = FORM ? p : powAny(p, G.zeta[z]);
+            const T q = FORM == 4 && z == 2 ? p1 * p : FORM ? p : powAny(p, G.zeta[z]);
             acc[l * Z + z] += c0 * q;
             if constexpr (TWO) acc[(2 + l) * Z + z] += c1 * q;
         }
@@ -999,8 +1008,9 @@ __device__ __forceinline__ void forcesStep(ForcesStage<T, CAP>& S, GroupCoef<T> 
         for (int z = 0; z < Z; ++z)
         {
             if (FORM == 0 && !(G.levels >> z & 1)) continue;
-            // a = p^(zeta - 1): 1, p, p^3, p^7, p^15 for the powers of two
-            if (FORM && z > 0)
+            // a = p^(zeta - 1): 1, p, p^3, p^7, p^15 for the powers of two, 1, p, p^2, p^3 for 1 to 4
+            if (FORM == 4 && z > 0) a = z == 1 ? p : a * p;
+            else if (FORM && z > 0)
             {
                 a = z == 1 ? p : a * sq;
                 sq = sq * sq;

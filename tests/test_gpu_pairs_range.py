@@ -1,8 +1,9 @@
 """The ends of the pair kernels' range of functions (sf_pairs.cuh): zeta up to
-32, Gaussians that underflow inside the cutoff (eta r^2 log2 e beyond the
-exponent range of a double, shifted and not, radial, narrow and wide) and
-shifts far out.  They run there (no candidate_masks stage, which only the
-general kernels have), with the C restatement's energies and forces.
+32, groups with zeta 1 to 4 alone and beside others, Gaussians that underflow
+inside the cutoff (eta r^2 log2 e beyond the exponent range of a double,
+shifted and not, radial, narrow and wide) and shifts far out.  They run there
+(no candidate_masks stage, which only the general kernels have), with the C
+restatement's energies and forces.
 
 Tolerances: those of the other parity tests, 1e-10 of the energy and of the
 largest force component."""
@@ -22,6 +23,9 @@ PLAIN = [(3, 0.01, 1, 4)]
 FORMS = {
     "zeta31": (RADIAL, PLAIN + [(3, 0.01, 1, 31), (9, 0.01, -1, 31)]),
     "zeta32": (RADIAL, PLAIN + [(3, 0.01, 1, 32), (3, 0.01, -1, 32), (9, 0.02, 1, 32), (9, 0.02, 1, 16)]),
+    "cubic": (RADIAL, [(3, e, la, z) for e in (0.01, 0.03) for la in (-1, 1) for z in (1, 3)] +
+              [(9, 0.02, 0.5, z) for z in (2, 3, 4)]),
+    "cubic_beside": (RADIAL, [(3, 0.01, la, z) for la in (-1, 1) for z in (3, 4)] + [(9, 0.02, 1, 7), (9, 0.05, -1, 3)]),
     "at_1000": (RADIAL + [(4.8, 0.0), (4.82, 0.0)], PLAIN),
     "wide_radial": (RADIAL + [(6.0, 0.0), (20.0, 0.0), (30.0, 2.0)], PLAIN),
     "far_shift": (RADIAL + [(2.0, 9.0), (4.0, 6.0), (3.0, 11.5)], PLAIN),
