@@ -773,9 +773,10 @@ n2p2_status n2p2_device_fma_peak(int device, double* fp64Tflops, double* fp32Tfl
         cudaCheck(cudaSetDevice(device), "cudaSetDevice");
         cudaDeviceProp p{};
         cudaCheck(cudaGetDeviceProperties(&p, device), "cudaGetDeviceProperties");
+        const LaunchErrors errors;
         if (fp64Tflops) *fp64Tflops = measureFmaPeak(1, p.multiProcessorCount);
         if (fp32Tflops) *fp32Tflops = measureFmaPeak(0, p.multiProcessorCount);
-        cudaCheck(cudaGetLastError(), "fma probe");
+        errors.check("fma probe");
     });
 }
 

@@ -1353,7 +1353,7 @@ void Batch::symmetryFunctionPass(int pass, int precision, int variant)
 // The kernel sequence of one evaluation (Mode::evaluateNNP, Mode.cpp:2029-2077).
 void Batch::record(int flags, int precision, int checkExtrapolation, std::vector<Mark>* marks, int stages)
 {
-    cudaGetLastError();   // an error another library's call left on this thread is not these launches'
+    const LaunchErrors errors;
     DevModel const& m = dmodel_.view;
     const bool sfOnly = (flags & EVAL_SF_ONLY) != 0;
     const bool forces = (flags & EVAL_FORCES) != 0 && !sfOnly;
@@ -1469,7 +1469,7 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
         launches += 1;
         mark("gather_forces");
     }
-    cudaCheck(cudaGetLastError(), "kernel launch");
+    errors.check("kernel launch");
     if (whole) launches_ = launches;
 }
 
@@ -1614,6 +1614,7 @@ Batch::TuneResult Batch::autotune(int precision, int checkExtrapolation, bool us
         // fill every pass input (neighbour data, dE/dG) once, then time the passes alone
         record(EVAL_FORCES, precision, checkExtrapolation);
         pendingVerify_ = true;
+        const LaunchErrors errors;
         cudaEvent_t e0, e1;
         cudaCheck(cudaEventCreate(&e0), "event");
         cudaCheck(cudaEventCreate(&e1), "event");
@@ -1637,7 +1638,7 @@ Batch::TuneResult Batch::autotune(int precision, int checkExtrapolation, bool us
             }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        cudaCheck(cudaGetLastError(), "autotune");
+        errors.check("autotune");
         r.values = (int)(std::min_element(r.valuesMs, r.valuesMs + kSFShapeCount) - r.valuesMs);
         r.forces = (int)(std::min_element(r.forcesMs, r.forcesMs + kSFShapeCount) - r.forcesMs);
         // the passes ran with every shape; results are identical whichever ran last
@@ -2090,8 +2091,9 @@ void Batch::sfStatistics(int64_t* counts, double* stats)
     double* partial = devAlloc<double>(pool_, (size_t)ne * maxChunks * 4 * maxSF, tmp);
     double* result = devAlloc<double>(pool_, (size_t)ne * 4 * maxSF, tmp);
     cudaCheck(cudaMemsetAsync(result, 0, sizeof(double) * (size_t)ne * 4 * maxSF, stream_), "memset");
+    const LaunchErrors errors;
     launchSFStatistics(dmodel_.view, v_, ne, maxChunks, maxSF, partial, result, stream_);
-    cudaCheck(cudaGetLastError(), "statistics launch");
+    errors.check("statistics launch");
     cudaCheck(cudaMemcpyAsync(stats, result, sizeof(double) * (size_t)ne * 4 * maxSF, cudaMemcpyDeviceToHost, stream_),
               "statistics D2H");
     synchronize();

@@ -282,6 +282,7 @@ void neighborListNoAlloc(const double* positions, int64_t numAtoms, const double
     cudaCheck(cudaMemsetAsync(cellCount, 0, sizeof(int) * cells, st), "memset");
     cudaCheck(cudaMemsetAsync(status, 0, sizeof(int) * 8, st), "memset");
     const int blocks = (N + 127) / 128;
+    const LaunchErrors errors;
     kNaAssign<<<blocks, 128, 0, st>>>(N, s, positions, atomCell, atomSlot, cellCount, status);
     launchExclusiveScan((int)cells, cellCount, cellStart64, tiles, nullptr, st);
     kNaScatter<<<blocks, 128, 0, st>>>(N, atomCell, atomSlot, cellStart64, cellAtoms);
@@ -292,7 +293,7 @@ void neighborListNoAlloc(const double* positions, int64_t numAtoms, const double
     launchExclusiveScan(N, count, offsets, tiles, nullptr, st);
     kNaSearch<1><<<wblocks, 128, 0, st>>>(N, rc2, s, positions, atomCell, cellStart64, cellCount, cellAtoms, count,
                                           offsets, capacity, index, image, d, dr, status);
-    cudaCheck(cudaGetLastError(), "kernel launch");
+    errors.check("kernel launch");
     // Recorded into the caller's graph: no host copy and no wait (neither may be captured); the
     // count and the limit checks are read after a replay by neighborListNoAllocStatus.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;

@@ -175,8 +175,11 @@ void cutoffFunctionValues(int type, double rc, double alpha, int fp32, const dou
     double* d = nullptr;
     cudaCheck(cudaMalloc(&d, sizeof(double) * 3 * (size_t)n), "cudaMalloc");
     cudaCheck(cudaMemcpy(d, r, sizeof(double) * (size_t)n, cudaMemcpyHostToDevice), "H2D");
+    const cudaError_t before = cudaPeekAtLastError();   // the caller's, as in LaunchErrors
     kCutoffValues<<<(int)std::min<int64_t>((n + 255) / 256, 1024), 256>>>(c, fp32, d, n, d + n, d + 2 * n);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = cudaPeekAtLastError();
+    if (e == before) e = cudaSuccess;
+    else cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpy(f, d + n, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(df, d + 2 * n, sizeof(double) * (size_t)n, cudaMemcpyDeviceToHost);
     cudaFree(d);

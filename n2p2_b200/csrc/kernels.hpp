@@ -87,6 +87,25 @@ void inverseBoxOf(double const* box, double* invbox);
 // Throws std::runtime_error("CUDA error in ...") on failure.
 void cudaCheck(cudaError_t e, char const* what);
 
+// Launch errors since construction.  The runtime holds one pending error per
+// thread: one that the caller or another library left there earlier is neither
+// taken for these launches' own nor cleared.  (A launch that fails with the
+// very error that was pending goes unnoticed.)
+class LaunchErrors
+{
+public:
+    void check(char const* what) const
+    {
+        const cudaError_t e = cudaPeekAtLastError();
+        if (e == before_) return;
+        cudaGetLastError();
+        cudaCheck(e, what);
+    }
+
+private:
+    cudaError_t before_ = cudaPeekAtLastError();
+};
+
 // Raise a kernel's dynamic shared-memory limit to `bytes` on the current
 // device (a no-op when an earlier call already set as much).
 void setDynamicSmemOnce(const void* kernel, size_t bytes);

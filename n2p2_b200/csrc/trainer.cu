@@ -582,6 +582,7 @@ void Trainer::step(Batch& batch, const double* energiesPhys, const double* force
     const int S = batch.numStructures(), N = batch.numAtoms();
     if (N == 0) throw std::runtime_error("ERROR: no structures set.\n");
     cudaStream_t st = batch.stream();
+    const LaunchErrors errors;
     batch.evaluate(EVAL_FORCES | EVAL_STORE_DGDR | EVAL_NO_GRAPH, PREC_FP64, 0);
     BatchView const& b = batch.view();
     reserve(S, N, b.gStride);
@@ -601,13 +602,13 @@ void Trainer::step(Batch& batch, const double* energiesPhys, const double* force
     kSFAdjoint<<<blocks, kTrainWarps * 32, 0, st>>>(m, b, 0, N, u_, g_);
     kParamGrad<true><<<blocks, kTrainWarps * 32, 0, st>>>(m, b, 0, N, aStruct_, 0.0, g_, P_, gradPart_, nullptr);
     kReduceGrad<<<(P_ + 7) / 8, 1024, 0, st>>>(gradPart_, warps_, P_, grad_);
-    cudaCheck(cudaGetLastError(), "trainer launch");
+    errors.check("trainer launch");
     if (update)
     {
         const double eta = eta0_ * std::sqrt(1.0 - beta2t_) / (1.0 - beta1t_);
         kAdam<<<(P_ + tb - 1) / tb, tb, 0, st>>>(P_, grad_, m_, v_, dmodel_.weightsDevice(), dmodel_.weightsTDevice(),
                                                  dmodel_.transIndexDevice(), beta1_, beta2_, eta, eps_);
-        cudaCheck(cudaGetLastError(), "adam launch");
+        errors.check("adam launch");
         beta1t_ *= beta1_;
         beta2t_ *= beta2_;
         ++steps_;
@@ -1330,6 +1331,7 @@ void Training::setGradientAdam(double eta, double beta1, double beta2, double ep
 // Jacobians carry the force weight.
 void Training::observation(int property, int s, int a, int c, int t, bool accumulate, bool last, int column)
 {
+    const LaunchErrors errors;
     const int acc = accumulate ? 1 : 0;
     double* H = H_ + (size_t)column * P_;   // the full Jacobian keeps one column per observation
     double* xi = xi_ + 2 * column;
@@ -1361,7 +1363,7 @@ void Training::observation(int property, int s, int a, int c, int t, bool accumu
         launchChained(kReduceSlices, (P_ + 31) / 32 + 1, 256, st, gradPart_, fw, P_, H, last ? forceWeight_ : 1.0, acc,
                       ObsError{predPart_, fRef_, k, forceWeight_, xi, err_ + t});
     }
-    cudaCheck(cudaGetLastError(), "observation launch");
+    errors.check("observation launch");
 }
 
 // The updaters' step with the observation in H_ / xi_: one updater over all
@@ -1369,6 +1371,7 @@ void Training::observation(int property, int s, int a, int c, int t, bool accumu
 // (element strategy), each with its share of the error.
 void Training::step(int property, int s, int a, int m)
 {
+    const LaunchErrors errors;
     cudaStream_t st = set_.stream();
     double* w = dmodel_.weightsDevice();
     double* wT = dmodel_.weightsTDevice();
@@ -1482,7 +1485,7 @@ void Training::step(int property, int s, int a, int m)
         beta1t_ *= beta1_;
         beta2t_ *= beta2_;
     }
-    cudaCheck(cudaGetLastError(), "updater launch");
+    errors.check("updater launch");
     ++numUpdates_;
 }
 
@@ -1507,9 +1510,10 @@ void Training::setUpdateStrategy(int strategy)
 void Training::initKalman(double epsilon)
 {
     if (!Pm_) Pm_ = tAlloc<double>((size_t)P_ * P_);
+    const LaunchErrors errors;
     for (Block const& B : blocks_)
         kKalmanInit<<<sms_ * 8, 256, 0, set_.stream()>>>(Pm_ + B.pOffset, B.count, 1.0 / epsilon);
-    cudaCheck(cudaGetLastError(), "kalman init");
+    errors.check("kalman init");
     pending_ = false;
     pendingRank_ = 1;
     cudaCheck(cudaMemsetAsync(Kb_[cur_], 0, sizeof(double) * P_ * kMaxObs, set_.stream()), "memset");
@@ -1687,13 +1691,14 @@ void Training::observe(int property, int structure, int atom, int component, dou
 void Training::flushKalman()
 {
     if (!pending_) return;
+    const LaunchErrors errors;
     for (Block const& B : blocks_)
     {
         dim3 grid((B.count + 255) / 256, B.count);
         kKalmanP<<<grid, 256, 0, set_.stream()>>>(Pm_ + B.pOffset, Kb_[cur_] + B.begin, Xb_[cur_] + B.begin, B.count,
                                                   pendingScale_, pendingQ_, pendingRank_, P_);
     }
-    cudaCheck(cudaGetLastError(), "kalman flush");
+    errors.check("kalman flush");
     pending_ = false;
 }
 
