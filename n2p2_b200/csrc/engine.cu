@@ -1394,7 +1394,7 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
             launches += 1;
             mark("prepare_positions");
             launchNeighborBuild(v_, model_.maxCutoffRadius * model_.maxCutoffRadius, stream_);
-            launches += 3 + 3 + 1 + 1 + 1 + 3 + 1 + 1 + 1;
+            launches += 1 + 3 + 1 + 1 + 1 + 3 + 1 + 1 + 1;   // the two scans are three each
             mark("neighbor_list");
         }
         launchCutoffValues(m, v_, sms_, stream_);
@@ -1419,13 +1419,13 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
         if (stored)
         {
             launchSFDerivatives(m, dmodel_.pairTable, v_, sms_, stream_);
-            launches += 2;
+            launches += m.pairForm ? 3 : 2;   // the tiers
             mark("sf_derivatives");
         }
         else
         {
             symmetryFunctionPass(0, precision, sfShape_[0][precision]);
-            launches += 2;
+            launches += m.pairForm ? 3 : 2;
             if (m.numCompactGroups > 0) launches += launchCompactValues(m, v_, sms_, stream_);
             mark("sf_values");
         }
@@ -1460,7 +1460,7 @@ void Batch::record(int flags, int precision, int checkExtrapolation, std::vector
         else
         {
             symmetryFunctionPass(1, precision, sfShape_[1][precision]);
-            launches += 2;
+            launches += m.pairForm ? 3 : 2;
             if (m.numCompactGroups > 0) launches += launchCompactForces(m, v_, sms_, stream_);
             mark("sf_forces");
         }
@@ -1755,6 +1755,26 @@ void Batch::calculateForces()
     stage_.forces = true;
 }
 
+namespace {
+
+int kernelNodes(cudaGraph_t graph)
+{
+    size_t n = 0;
+    cudaCheck(cudaGraphGetNodes(graph, nullptr, &n), "graph nodes");
+    std::vector<cudaGraphNode_t> nodes(n);
+    cudaCheck(cudaGraphGetNodes(graph, nodes.data(), &n), "graph nodes");
+    int kernels = 0;
+    for (cudaGraphNode_t node : nodes)
+    {
+        cudaGraphNodeType type;
+        cudaCheck(cudaGraphNodeGetType(node, &type), "graph node");
+        kernels += type == cudaGraphNodeTypeKernel ? 1 : 0;
+    }
+    return kernels;
+}
+
+} // namespace
+
 void Batch::evaluate(int flags, int precision, int checkExtrapolation)
 {
     if (N_ == 0) throw std::runtime_error("ERROR: no structures set.\n");
@@ -1843,10 +1863,12 @@ void Batch::evaluate(int flags, int precision, int checkExtrapolation)
         }
         cudaCheck(cudaStreamEndCapture(stream_, &graph), "end capture");
         cudaCheck(cudaGraphInstantiate(&graphExec_, graph, 0), "graph instantiate");
+        graphLaunches_ = kernelNodes(graph);
         cudaGraphDestroy(graph);
         graphKey_ = key;
     }
     cudaCheck(cudaGraphLaunch(graphExec_, stream_), "graph launch");
+    launches_ = graphLaunches_;
     pendingVerify_ = true;
 }
 

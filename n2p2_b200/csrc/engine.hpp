@@ -310,7 +310,8 @@ private:
     bool dgdrAllocated_ = false;
     cudaGraphExec_t graphExec_ = nullptr;
     int graphKey_ = -1;
-    int launches_ = 0;
+    int launches_ = 0;                // kernels of the last evaluation
+    int graphLaunches_ = 0;           // kernels of the captured graph
     int sfShape_[2][2] = {{1, 1}, {1, 1}};   // [values, forces][precision]: first-tier shape variant
     bool tuned_[2] = {false, false};
     TuneResult lastTune_[2];
