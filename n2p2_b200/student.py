@@ -566,9 +566,19 @@ def benchmark(student_dir, teacher_dir, num=2048, seed=97, steps=3, warmup=2, de
     of the training recipe (own seed).  Both forms are timed the same way:
     one evaluation plus the energies and forces read back, per step."""
     structs = training_structures(num, seed)
+    teacher = load_mode(teacher_dir, device, extrapolation=True)
+    smode = load_mode(student_dir, device, extrapolation=True)
+    try:
+        return _benchmark(smode, teacher, structs, seed, steps, warmup, monitor)
+    finally:   # with all their batches: a mode and its batches refer to each other
+        smode.close()
+        teacher.close()
+
+
+def _benchmark(smode, teacher, structs, seed, steps, warmup, monitor):
+    num = len(structs)
     natoms = sum(s.numAtoms for s in structs)
     apa = [s.numAtoms for s in structs]
-    teacher = load_mode(teacher_dir, device, extrapolation=True)
     tb = teacher.batch(structs)
     tb.setPositions(_positions(structs))
 
@@ -586,7 +596,6 @@ def benchmark(student_dir, teacher_dir, num=2048, seed=97, steps=3, warmup=2, de
     starts = np.concatenate([[0], np.cumsum(apa)])
     teacher_in_range = np.add.reduceat(per_atom, starts[:-1]) == 0
 
-    smode = load_mode(student_dir, device, extrapolation=True)
     ev = StudentEvaluator(smode, teacher, structs, monitor=monitor, seed=seed)
     for _ in range(warmup):
         Es, Fs, flagged = ev.evaluate()
