@@ -166,6 +166,11 @@ def run_reference(args):
     rank, world, _ = dist_env()
     if rank != 0:
         return
+    from oracle import ref
+    if not ref.available(fast=True):
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref/libnnpref_fast.so is not built: the "
+                          "reference's sources are not on this machine"}), flush=True)
+        return
     structs = workload(args.boxes, args.seed)
     threads = host_threads()
     sample, natoms = cpu_sample(structs, threads)
