@@ -508,11 +508,24 @@ __global__ void __launch_bounds__(128, 2) kCompactForces(DevModel model, BatchVi
 constexpr int kWideRows = kCompactStageRows;   // radial parts per chunk
 constexpr int kWideCols = kCompactStageCols;   // angular parts per chunk
 // Two shapes of a block: four warps for atoms with up to kWideCap neighbours
-// (more run the direct kernels), one warp for those with up to kSmallCap
-// (molecules: a pair list of a few batches; 15 neighbours make 105 pairs, and
-// four warps per atom spent their time in barriers).
+// (more run the direct kernels), one warp for atoms with few (molecules: a pair
+// list of a few batches; 15 neighbours make 105 pairs, and four warps per atom
+// spent their time in barriers).  Few are up to smallCap where the whole batch
+// has no more and fills the SMs with one-warp blocks, else kSmallMixed: an
+// atom's pairs take one warp four times as long, and beside larger atoms, or
+// with few blocks, that is the kernel's time.  The one-warp kernel runs beside
+// the four-warp kernel (programmatic launch; it ends after it).
+// 27 models of other cores than p2, G and forces: 7,200 atoms of 30 to 110
+// neighbours 204 ms in all (one warp up to 64 neighbours in every batch, launched
+// first: 226; no one-warp blocks: 207); 3,840 atoms in molecules of 12, 33 and 62
+// 12.3, 24.0 and 33.7 ms (12.5, 24.1, 34.7; 18.7, 26.8, 35.4); one box of 192
+// 25.7 (26.2; 26.2).
 constexpr int kWideCap = 256, kWideWarps = 4;
-constexpr int kSmallCap = 64, kSmallWarps = 1;
+constexpr int kSmallCap = 64, kSmallWarps = 1, kSmallMixed = 20;
+
+// The weighted types pair all neighbours of an atom, the others two elements'.
+__host__ __device__ constexpr int smallCap(int type) { return type >= 24 ? 32 : kSmallCap; }
+
 constexpr int kCellStride = 8;  // G pass cell sums: row r, column a at r * 8 + a
 constexpr int kTileStride = 36; // per-warp tile: 32 pairs per row, padded against bank conflicts
 
@@ -668,11 +681,14 @@ __device__ __forceinline__ void blockSync()
     else __syncthreads();
 }
 
-// The block's atoms: those of the type with lower < n <= CAP neighbours,
-// found blockDim.x at a time; f(i) runs on the whole block.
+// The block's atoms: those of the type with up to `few` neighbours (one-warp
+// shape) or more, up to CAP, found blockDim.x at a time; f(i) runs on the whole
+// block.  few: `few` where no atom of the batch has more, else kSmallMixed.
 template <int TYPE, int CAP, int WARPS, typename F>
-__device__ __forceinline__ void forTypeAtoms(DevModel const& model, BatchView const& b, int lower, F f)
+__device__ __forceinline__ void forTypeAtoms(DevModel const& model, BatchView const& b, int few, F f)
 {
+    if (b.status->maxNeighbors > few) few = kSmallMixed;
+    const int lower = CAP == kSmallCap ? -1 : few, upper = CAP == kSmallCap ? few : CAP;
     __shared__ unsigned todo[WARPS];
     constexpr int T = WARPS * 32;
     const int tid = threadIdx.x;
@@ -685,7 +701,7 @@ __device__ __forceinline__ void forTypeAtoms(DevModel const& model, BatchView co
         {
             const int64_t off = b.nbrOffset[i], end = b.nbrOffset[i + 1];
             const int n = (int)(end - off);
-            mine = end <= b.nbrCapacity && n > lower && n <= CAP;
+            mine = end <= b.nbrCapacity && n > lower && n <= upper;
             if (mine)
             {
                 DevElement const& E = model.el[b.elem[i]];
@@ -887,7 +903,7 @@ __device__ __forceinline__ unsigned long long walkMasks(WideSmem const& S, int u
 
 template <int TYPE, int CORE, int CAP, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
-    kCompactWideValues(const __grid_constant__ DevModel model, const __grid_constant__ BatchView b, int rows, int lower)
+    kCompactWideValues(const __grid_constant__ DevModel model, const __grid_constant__ BatchView b, int rows, int few)
 {
     constexpr bool WEIGHTED = TYPE >= 24;
     constexpr bool NARROW = TYPE == 21 || TYPE == 24;
@@ -900,7 +916,8 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
     double* AT = PT + TR * kTileStride;
     double* cw = S.cell + warp * cellCount<NARROW>();
     const int g4 = lane >> 2, t4 = lane & 3;              // mma fragment row / column of the lane
-    forTypeAtoms<TYPE, CAP, WARPS>(model, b, lower, [&](int i) {
+    if (CAP != kSmallCap) cudaTriggerProgrammaticLaunchCompletion();
+    forTypeAtoms<TYPE, CAP, WARPS>(model, b, few, [&](int i) {
         DevElement const& E = model.el[b.elem[i]];
         const int64_t off = b.nbrOffset[i];
         const int n = (int)(b.nbrOffset[i + 1] - off);
@@ -1044,6 +1061,7 @@ __global__ void __launch_bounds__(WARPS * 32, 16 / WARPS)
                 }
         }
     });
+    if (CAP == kSmallCap) cudaGridDependencySynchronize();
 }
 
 // G pass of the wide types without a narrow window where the grid fits
@@ -1056,7 +1074,7 @@ constexpr int kGridRows = 10, kGridCols = 6;
 
 template <int TYPE, int ROWS, int CAP, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
-    kCompactGridValues(const __grid_constant__ DevModel model, const __grid_constant__ BatchView b, int rows, int lower)
+    kCompactGridValues(const __grid_constant__ DevModel model, const __grid_constant__ BatchView b, int rows, int few)
 {
     constexpr bool WEIGHTED = TYPE >= 24;
     constexpr int T = WARPS * 32, CELLS = ROWS * kGridCols;
@@ -1065,7 +1083,8 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double* scratch = S.tile + warp * tileDoubles<false>();
     double* cw = S.cell + warp * cellCount<false>();
-    forTypeAtoms<TYPE, CAP, WARPS>(model, b, lower, [&](int i) {
+    if (CAP != kSmallCap) cudaTriggerProgrammaticLaunchCompletion();
+    forTypeAtoms<TYPE, CAP, WARPS>(model, b, few, [&](int i) {
         DevElement const& E = model.el[b.elem[i]];
         const int64_t off = b.nbrOffset[i];
         const int n = (int)(b.nbrOffset[i + 1] - off);
@@ -1143,11 +1162,12 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
             blockSync<WARPS>();
         }
     });
+    if (CAP == kSmallCap) cudaGridDependencySynchronize();
 }
 
 template <int TYPE, int CORE, int COLS, int CAP, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
-    kCompactWideForces(const __grid_constant__ DevModel model, const __grid_constant__ BatchView b, int rows, int lower)
+    kCompactWideForces(const __grid_constant__ DevModel model, const __grid_constant__ BatchView b, int rows, int few)
 {
     constexpr bool WEIGHTED = TYPE >= 24;
     constexpr bool NARROW = TYPE == 21 || TYPE == 24;
@@ -1158,7 +1178,8 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     double* hw = S.h + warp * 3 * CAP;   // this warp's force array
     for (int k = tid; k < WARPS * 3 * CAP; k += T) S.h[k] = 0.0;
-    forTypeAtoms<TYPE, CAP, WARPS>(model, b, lower, [&](int i) {
+    if (CAP != kSmallCap) cudaTriggerProgrammaticLaunchCompletion();
+    forTypeAtoms<TYPE, CAP, WARPS>(model, b, few, [&](int i) {
         DevElement const& E = model.el[b.elem[i]];
         const int64_t off = b.nbrOffset[i];
         const int n = (int)(b.nbrOffset[i + 1] - off);
@@ -1394,6 +1415,7 @@ __global__ void __launch_bounds__(WARPS * 32, 12 / WARPS)
         }
         blockSync<WARPS>();
     });
+    if (CAP == kSmallCap) cudaGridDependencySynchronize();
 }
 
 } // namespace
@@ -1427,10 +1449,21 @@ int launchAngular(DevModel const& m, BatchView const& b, int sms, cudaStream_t s
     const int rows = std::max(1, std::min(m.compactRows, kWideRows));
     // resident blocks: the launch bound, or fewer when the stage is larger (228 KB of shared memory
     // per SM, 1 KB of it reserved per block)
-    auto staged = [&](auto kernel, size_t smem, int warps, int perSM, int lower) {
+    const int few = b.N >= 12 * sms ? smallCap(TYPE) : kSmallMixed;   // 12 one-warp blocks per SM
+    auto staged = [&](auto kernel, size_t smem, int warps, int perSM) {
         perSM = std::max(1, std::min(perSM, (int)(233472 / (smem + 1024))));
         setDynamicSmemOnce(reinterpret_cast<const void*>(kernel), smem);
-        kernel<<<std::max(1, std::min(b.N, sms * perSM)), warps * 32, smem, st>>>(m, b, rows, lower);
+        cudaLaunchAttribute beside{};
+        beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        beside.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(std::max(1, std::min(b.N, sms * perSM)));
+        cfg.blockDim = dim3(warps * 32);
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = st;
+        cfg.attrs = &beside;
+        cfg.numAttrs = warps == kSmallWarps ? 1 : 0;   // launched second, beside the four-warp shape
+        cudaCheck(cudaLaunchKernelEx(&cfg, kernel, m, b, rows, few), "compact launch");
     };
     const size_t large = wideSmemBytes<kWideCap, kWideWarps>(rows, FORCES, NARROW);
     const size_t small = wideSmemBytes<kSmallCap, kSmallWarps>(rows, FORCES, NARROW);
@@ -1440,8 +1473,8 @@ int launchAngular(DevModel const& m, BatchView const& b, int sms, cudaStream_t s
         // six angular parts per chunk where the model has no more (the SCAN and QM9 groups)
         auto both = [&](auto core, auto cols) {
             constexpr int C = decltype(core)::value, A = decltype(cols)::value;
-            staged(kCompactWideForces<TYPE, C, A, kSmallCap, kSmallWarps>, small, kSmallWarps, 12, -1);
-            staged(kCompactWideForces<TYPE, C, A, kWideCap, kWideWarps>, large, kWideWarps, 3, kSmallCap);
+            staged(kCompactWideForces<TYPE, C, A, kWideCap, kWideWarps>, large, kWideWarps, 3);
+            staged(kCompactWideForces<TYPE, C, A, kSmallCap, kSmallWarps>, small, kSmallWarps, 12);
         };
         using Poly2 = std::integral_constant<int, kCorePoly2>;
         using Any = std::integral_constant<int, 0>;
@@ -1464,8 +1497,8 @@ int launchAngular(DevModel const& m, BatchView const& b, int sms, cudaStream_t s
             {
                 auto grid = [&](auto cells) {
                     constexpr int R = decltype(cells)::value;
-                    staged(kCompactGridValues<TYPE, R, kSmallCap, kSmallWarps>, small, kSmallWarps, 12, -1);
-                    staged(kCompactGridValues<TYPE, R, kWideCap, kWideWarps>, large, kWideWarps, 3, kSmallCap);
+                    staged(kCompactGridValues<TYPE, R, kWideCap, kWideWarps>, large, kWideWarps, 3);
+                    staged(kCompactGridValues<TYPE, R, kSmallCap, kSmallWarps>, small, kSmallWarps, 12);
                 };
                 if (m.compactRows <= 6) grid(std::integral_constant<int, 6>{});
                 else if (m.compactRows <= 9) grid(std::integral_constant<int, 9>{});
@@ -1476,8 +1509,8 @@ int launchAngular(DevModel const& m, BatchView const& b, int sms, cudaStream_t s
         {
             auto both = [&](auto core) {
                 constexpr int C = decltype(core)::value;
-                staged(kCompactWideValues<TYPE, C, kSmallCap, kSmallWarps>, small, kSmallWarps, 16, -1);
-                staged(kCompactWideValues<TYPE, C, kWideCap, kWideWarps>, large, kWideWarps, NARROW ? 3 : 4, kSmallCap);
+                staged(kCompactWideValues<TYPE, C, kWideCap, kWideWarps>, large, kWideWarps, NARROW ? 3 : 4);
+                staged(kCompactWideValues<TYPE, C, kSmallCap, kSmallWarps>, small, kSmallWarps, 16);
             };
             if (poly2) both(std::integral_constant<int, kCorePoly2>{});
             else both(std::integral_constant<int, 0>{});
