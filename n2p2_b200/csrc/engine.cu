@@ -852,11 +852,11 @@ void DeviceModel::upload(Model const& m)
     // Networks of the mixed form: a choice of the model alone, so that a structure's energy depends
     // neither on its batch nor on a rank's number of atoms (the tensor-core form is off by up to
     // 0.1 meV per atom, part of it systematic).  Up to kExactParameters per element the FP64 kernels:
-    // 1,701 parameters take them 23 to 26 us for 192 to 4,320 atoms (tensor cores 50: a chain of
-    // four products and their waits, however few the tiles) and 520 us for 138 k (344), of whole
-    // calls of 200 us and 11.2 ms; 945 parameters 20 us (35) and 430 us (217).  Above it the tensor cores:
-    // 4,369 parameters 37 us (70) for 192 atoms, but 995 (492) of 11.4 ms for 138 k; 6,849 43 (88)
-    // and 1,165 (621).
+    // 1,701 parameters take them 23 to 29 us for 192 to 4,320 atoms (tensor cores 50: a chain of
+    // four products and their waits, however few the tiles) and 389 us for 138 k (344), of whole
+    // calls of 200 us and 11.1 ms; 945 parameters 19 us (35) and 318 us (217).  Above it the tensor cores:
+    // 4,369 parameters 37 us (70) for 192 atoms, but 991 (485) of 11.3 ms for 138 k; 6,849 43 (88)
+    // and 1,163 (621).
     constexpr int kExactParameters = 2048;
     bool small = true;
     for (int e = 0; e < v.numElements; ++e)

@@ -187,10 +187,9 @@ namespace {
 // neuron, reading a weight once (through the read-only cache: every block of
 // an element reads the same matrices) for UNIT fused multiply-adds.  Every sum
 // runs over the reduction index in ascending order, as in propagateLayer.
-// Bound by latency and the weights' loads, so by the blocks that fit an SM: only the
-// first activation buffer has the inputs' width, the other three the hidden layers'
-// (40-25-25-1 networks of 133 k atoms 527 -> 380 us; 354-30-20-1 networks, which a
-// tile did not hold before, 151 us by kNetworkFP64 -> 96 us for 4,096 atoms).
+// Bound by latency and the weights' loads.  Only the first activation buffer has the
+// inputs' width, the other three the hidden layers', so that wide inputs fit a tile
+// (354-30-20-1 networks of 4,096 atoms: 151 us by kNetworkFP64, 96 us so).
 constexpr int kNetThreads = 128;
 
 // Row of a tile of TILE atoms: padded by four against bank conflicts (rows stay 32-byte aligned).
@@ -601,10 +600,13 @@ void launchNetworkFP64(DevModel const& m, BatchView const& b, int derivatives, i
         t16 += (b.elemBegin[e + 1] - b.elemBegin[e] + 15) / 16;
         t8 += (b.elemBegin[e + 1] - b.elemBegin[e] + 7) / 8;
     }
-    auto tiled = [&](auto kernel, size_t bytes, int tiles) {
+    // resident: blocks per SM that the kernel's registers allow (144 and 80 a thread).  A fourth block of
+    // the wide units per SM, which its shared memory would allow, waits for one of the three and makes
+    // the last wave: 40-25-25-1 networks of 133 k atoms 382 -> 526 us.
+    auto tiled = [&](auto kernel, size_t bytes, int tiles, int resident) {
         if (tiles == 0) return;
         setDynamicSmemOnce(reinterpret_cast<const void*>(kernel), bytes);
-        const int perSM = std::max(1, std::min(4, (int)(233472 / (bytes + 1024))));
+        const int perSM = std::max(1, std::min(resident, (int)(233472 / (bytes + 1024))));
         kernel<<<std::min(tiles, sms * perSM), kNetThreads, bytes, st>>>(m, b, derivatives);
     };
     constexpr size_t kTileBudget = 110 * 1024;
@@ -612,9 +614,9 @@ void launchNetworkFP64(DevModel const& m, BatchView const& b, int derivatives, i
     // of the serial activations per thread (192 atoms: 34 -> 18 us; 4,320 atoms: 39 -> 21 us; from one
     // tile of 32 per SM on the wide units' fewer weight loads win).  Every sum keeps its order.
     if (t32 < sms && (size_t)d8 * sizeof(double) <= kTileBudget)
-        return tiled(kNetworkTiled<8, 2>, (size_t)d8 * sizeof(double), t8);
-    if ((size_t)d32 * sizeof(double) <= kTileBudget) return tiled(kNetworkTiled<32, 8>, (size_t)d32 * sizeof(double), t32);
-    if ((size_t)d16 * sizeof(double) <= kTileBudget) return tiled(kNetworkTiled<16, 8>, (size_t)d16 * sizeof(double), t16);
+        return tiled(kNetworkTiled<8, 2>, (size_t)d8 * sizeof(double), t8, 4);
+    if ((size_t)d32 * sizeof(double) <= kTileBudget) return tiled(kNetworkTiled<32, 8>, (size_t)d32 * sizeof(double), t32, 3);
+    if ((size_t)d16 * sizeof(double) <= kTileBudget) return tiled(kNetworkTiled<16, 8>, (size_t)d16 * sizeof(double), t16, 3);
     size_t smem = sizeof(NNWarpSmem) * kNNWarps;
     setDynamicSmemOnce(reinterpret_cast<const void*>(kNetworkFP64), smem);
     int blocks = (b.N + kNNWarps - 1) / kNNWarps;
