@@ -130,7 +130,10 @@ void launchSFValuesF32(DevModel const& m, BatchView const& b, int sms, cudaStrea
 void launchSFForcesF32(DevModel const& m, BatchView const& b, int sms, cudaStream_t st);
 // The same passes for the models of the pair kernels (DevModel::pairForm;
 // sf_pairs.cuh); `variant` (0 .. kSFShapeCount - 1): the first tier's stage
-// capacity, 128, 160 or 192 neighbours.
+// capacity, 128, 160 or 192 neighbours.  A larger stage costs resident blocks,
+// a smaller one sends atoms to the next tier's 384: G of 33 k atoms takes 1.26
+// ms with 160 or 192 and 107 neighbours on average, 4.49 and 2.31 with 157, so
+// the autotuner chooses.
 constexpr int kSFShapeCount = 3;
 void launchPairValuesF64(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
 void launchPairValuesF32(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);

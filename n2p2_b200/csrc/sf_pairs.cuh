@@ -26,7 +26,7 @@
 // and 35 %), then the latency of dependent FP64 and shared-memory
 // instructions.  Per water atom (107 neighbours, 2548 narrow triplets, 8
 // members) the G pass executes 28.5 k warp instructions: 5.7 k staging, radial
-// functions and sums, 11 k candidates, 11.8 k triplets; the force pass 39.7 k.
+// functions and sums, 11 k candidates, 11.8 k triplets; the force pass 41 k.
 // A warp per atom (the former specialised kernels) took 56 k and 73 k: its
 // member grids had run-time exponents (selects and branches per factor) and
 // every triplet read 14 separate values.  256 water boxes (133 k atoms), FP64:
