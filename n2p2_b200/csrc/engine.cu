@@ -1004,6 +1004,7 @@ void Batch::setStructures(std::vector<StructureInput> const& s, const int* eleme
     pendingVerify_ = false;
     stage_ = StageState{};
     tuned_[0] = tuned_[1] = false;   // new workload: shapes come from the cache or are measured again
+    shapesSet_[0] = shapesSet_[1] = false;
 }
 
 // Atoms grouped by element (the tensor-core networks run per element).
@@ -1578,6 +1579,17 @@ std::string Batch::tuneKey(int precision)
     return buf;
 }
 
+// The first-tier shape for a batch whose largest count is maxNeighbors: `shape`, or the smallest that
+// holds it.  One atom beyond the stage costs a block of the next tier's kernel, whose latency is that of
+// the whole pass for few atoms (387 atoms, one with 135 neighbours: 163 us with 160, 327 to 440 with 128),
+// while a larger stage that is not needed costs under 0.1 % (kernels.hpp).
+int Batch::fittingShape(int shape, int maxNeighbors) const
+{
+    if (!dmodel_.view.pairForm || maxNeighbors > kSFShapeCapacity[kSFShapeCount - 1]) return shape;
+    while (maxNeighbors > kSFShapeCapacity[shape]) ++shape;
+    return shape;
+}
+
 void Batch::setShapes(int precision, int values, int forces)
 {
     if (precision < 0 || precision > 1 || values < 0 || values >= kSFShapeCount || forces < 0 ||
@@ -1585,7 +1597,7 @@ void Batch::setShapes(int precision, int values, int forces)
         throw std::invalid_argument("ERROR: shape variant out of range.\n");
     sfShape_[0][precision] = values;
     sfShape_[1][precision] = forces;
-    tuned_[precision] = true;
+    tuned_[precision] = shapesSet_[precision] = true;
     releaseGraph();
 }
 
@@ -1672,9 +1684,16 @@ Batch::TuneResult Batch::autotune(int precision, int checkExtrapolation, bool us
             std::rename(tmp.c_str(), path.c_str());   // atomic replace; a failed write leaves no cache
         }
     }
+    if (r.fromCache)   // measured on another batch of the class
+    {
+        const int most = status().maxNeighbors;
+        r.values = fittingShape(r.values, most);
+        r.forces = fittingShape(r.forces, most);
+    }
     sfShape_[0][precision] = r.values;
     sfShape_[1][precision] = r.forces;
     tuned_[precision] = true;
+    shapesSet_[precision] = false;
     lastTune_[precision] = r;
     releaseGraph();
     return r;
@@ -1884,6 +1903,15 @@ void Batch::verify()
         const int64_t stride = strideFor(st.maxNeighbors);
         strideWanted_ = (int64_t)N_ * stride <= 2 * capacity_ ? stride : 0;
     }
+    // Positions that outgrew the first tier's stage: later evaluations take the one that holds them.
+    if (!shapesSet_[lastPrecision_])
+        for (int pass = 0; pass < 2; ++pass)
+        {
+            int& shape = sfShape_[pass][lastPrecision_];
+            const int fit = fittingShape(shape, st.maxNeighbors);
+            if (fit != shape) releaseGraph();
+            shape = fit;
+        }
     if (st.totalNeighbors <= capacity_) return;
     // The lists outgrew the buffers sized at the first evaluation: size them
     // again and repeat the evaluation directly (the graph is recaptured at

@@ -314,6 +314,8 @@ private:
     int graphLaunches_ = 0;           // kernels of the captured graph
     int sfShape_[2][2] = {{1, 1}, {1, 1}};   // [values, forces][precision]: first-tier shape variant
     bool tuned_[2] = {false, false};
+    bool shapesSet_[2] = {false, false};     // by setShapes
+    int fittingShape(int shape, int maxNeighbors) const;
     TuneResult lastTune_[2];
     std::string tuneKey(int precision);
     DevicePool pool_;

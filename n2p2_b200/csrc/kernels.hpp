@@ -134,7 +134,7 @@ void launchSFForcesF32(DevModel const& m, BatchView const& b, int sms, cudaStrea
 // a smaller one sends atoms to the next tier's 384: G of 33 k atoms takes 1.26
 // ms with 160 or 192 and 107 neighbours on average, 4.49 and 2.31 with 157, so
 // the autotuner chooses.
-constexpr int kSFShapeCount = 3;
+constexpr int kSFShapeCount = 3, kSFShapeCapacity[kSFShapeCount] = {128, 160, 192};
 void launchPairValuesF64(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
 void launchPairValuesF32(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);
 void launchPairForcesF64(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant);

@@ -40,7 +40,7 @@ inline int tierBlocks(int N, int sms, int perSM)
 template <typename T, int CUT, int FORM>
 void pairValues(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant)
 {
-    const int cap0 = variant == 0 ? 128 : variant == 1 ? 160 : 192;
+    const int cap0 = kSFShapeCapacity[variant];
     if (variant == 0) pairValuesTier<T, 128, CUT, FORM, false>(m, gt, b, b.N, -1, 0, st);
     else if (variant == 1) pairValuesTier<T, 160, CUT, FORM, false>(m, gt, b, b.N, -1, 0, st);
     else pairValuesTier<T, 192, CUT, FORM, false>(m, gt, b, b.N, -1, 0, st);
@@ -51,7 +51,7 @@ void pairValues(DevModel const& m, DevPairTable const& gt, BatchView const& b, i
 template <typename T, int CUT, int FORM>
 void pairForces(DevModel const& m, DevPairTable const& gt, BatchView const& b, int sms, cudaStream_t st, int variant)
 {
-    const int cap0 = variant == 0 ? 128 : variant == 1 ? 160 : 192;
+    const int cap0 = kSFShapeCapacity[variant];
     if (variant == 0) pairForcesTier<T, 128, CUT, FORM, false>(m, gt, b, b.N, -1, st);
     else if (variant == 1) pairForcesTier<T, 160, CUT, FORM, false>(m, gt, b, b.N, -1, st);
     else pairForcesTier<T, 192, CUT, FORM, false>(m, gt, b, b.N, -1, st);
