@@ -1581,7 +1581,7 @@ std::string Batch::tuneKey(int precision)
 
 // The first-tier shape for a batch whose largest count is maxNeighbors: `shape`, or the smallest that
 // holds it.  One atom beyond the stage costs a block of the next tier's kernel, whose latency is that of
-// the whole pass for few atoms (387 atoms, one with 135 neighbours: 163 us with 160, 327 to 440 with 128),
+// the whole pass for few atoms (387 atoms, at most 135 neighbours: a replay takes 163 us with 160, 327 to 440 with 128),
 // while a larger stage that is not needed costs under 0.1 % (kernels.hpp).
 int Batch::fittingShape(int shape, int maxNeighbors) const
 {
